@@ -62,6 +62,7 @@ static void dfree(void* p) {
 static void free_level(ssg::DevLevel& d) {
   dfree(d.gf); dfree(d.bj); dfree(d.kdiag); dfree(d.dinv_p); dfree(d.dinv_h);
   dfree(d.mult); dfree(d.mask); dfree(d.D); dfree(d.S); dfree(d.Ar); dfree(d.Ap);
+  dfree(d.aff); dfree(d.w);
   dfree(d.gf32); dfree(d.dinv_p32); dfree(d.dss_ec); dfree(d.det); dfree(d.rho);
   d = ssg::DevLevel();
 }
@@ -264,6 +265,14 @@ static ssg_status upload_all(ssg_context* c) {
     }
     SSG_TRY(dupload(c, &d.gf, gf.data(), gf.size()));
     SSG_TRY(dupload(c, &d.bj, bj.data(), np));
+    {
+      std::vector<double> aff;
+      affine_metric(h, nel, aff);
+      if (!aff.empty()) {
+        SSG_TRY(dupload(c, &d.aff, aff.data(), aff.size()));
+        SSG_TRY(dupload(c, &d.w, h.w.data(), h.w.size()));
+      }
+    }
     SSG_TRY(dupload(c, &d.kdiag, kd.data(), np));
     SSG_TRY(dupload(c, &d.dinv_p, dp.data(), np));
     SSG_TRY(dalloc(c, &d.dinv_h, np));

@@ -45,14 +45,15 @@ namespace dev {
 // ax_element (kernels.cuh), shared with the cooperative level smoother
 // ---------------------------------------------------------------------------
 
-template <int N, typename T, bool HELM, bool FUSEP>
+template <int N, typename T, bool HELM, bool FUSEP, bool AFF>
 __global__ void __launch_bounds__(256, (N >= 10 ? 1 : 2)) k_ax(int nel, T* __restrict__ u,
                                                T* __restrict__ au,
                                                const T* __restrict__ gf, size_t npts,
                                                const double* __restrict__ bj,
                                                const double* __restrict__ Dg,
                                                const double* __restrict__ Sg,
-                                               double lambda, PUpdate pu, ScalarOp dop) {
+                                               double lambda, PUpdate pu, ScalarOp dop,
+                                               AffGeom ag) {
   using L = AxSmem<N>;
   if (FUSEP && pu.stop && *pu.stop != 0.0) return;   // uniform over the block
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -66,9 +67,10 @@ __global__ void __launch_bounds__(256, (N >= 10 ? 1 : 2)) k_ax(int nel, T* __res
   const T* z = FUSEP ? reinterpret_cast<const T*>(pu.z) : nullptr;
   const double beta = (FUSEP && !pu.first) ? *pu.beta : 0.0;
   const double c = (FUSEP && pu.c) ? *pu.c : 0.0;
-  const double pap = ax_element<N, T, HELM, FUSEP>(e, e < nel, i, j, sD, su, su + L::BLK,
+  const double pap = ax_element<N, T, HELM, FUSEP, AFF>(e, e < nel, i, j, sD, su, su + L::BLK,
                                                    su + 2 * L::BLK, u, au, gf, npts, bj,
-                                                   lambda, z, beta, c, pu.mask, pu.first != 0);
+                                                   lambda, z, beta, c, pu.mask, pu.first != 0,
+                                                   ag);
   if (FUSEP && pu.part) {
     __shared__ double sflat[256];
     finish_flat(pap, tid, nthr, pu.part, dop, sflat);
@@ -88,11 +90,11 @@ __global__ void __launch_bounds__(256, (N >= 10 ? 1 : 2)) k_ax(int nel, T* __res
 // per 16-byte load.  EPB elements per block fill about 256 threads.  Same
 // interface as k_ax (optional direction update and p . (A p)).
 // ---------------------------------------------------------------------------
-template <int N, typename T, bool HELM, bool FUSEP>
+template <int N, typename T, bool HELM, bool FUSEP, bool AFF>
 __global__ void __launch_bounds__(AxLine<N>::THREADS)
     k_axl(int nel, T* __restrict__ u, T* __restrict__ au, const T* __restrict__ gf,
           size_t npts, const double* __restrict__ bj, const double* __restrict__ Dg,
-          const double* __restrict__ Sg, double lambda, PUpdate pu, ScalarOp dop) {
+          const double* __restrict__ Sg, double lambda, PUpdate pu, ScalarOp dop, AffGeom ag) {
   using L = AxLine<N>;
   if (FUSEP && pu.stop && *pu.stop != 0.0) return;   // uniform over the block
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -103,9 +105,9 @@ __global__ void __launch_bounds__(AxLine<N>::THREADS)
   const double beta = (FUSEP && !pu.first) ? *pu.beta : 0.0;
   const double c = (FUSEP && pu.c) ? *pu.c : 0.0;
   double rdz = 0.0;
-  const double pap = axl_group<N, T, HELM, FUSEP>(
+  const double pap = axl_group<N, T, HELM, FUSEP, AFF>(
       e0, min(L::EPB, nel - e0), u, au, gf, npts, bj, lambda, z, beta, c, pu.mask,
-      pu.first != 0, sD, nullptr, nullptr, &rdz);
+      pu.first != 0, sD, nullptr, nullptr, &rdz, ag);
   if (FUSEP && pu.part) {
     __shared__ double sflat[AxLine<N>::THREADS];
     finish_flat(pap, threadIdx.x, blockDim.x, pu.part, dop, sflat);
@@ -935,38 +937,34 @@ int ax_epb(int n) {
   return kAxLine;
 }
 
-template <int N, typename T, bool HELM, bool FUSEP>
-static cudaError_t launch_ax_t(cudaStream_t s, int nel, int epb, T* u, T* au, const T* gf,
+// the plane-form (epb > 0 elements per block) or line-form (kAxLine) kernel
+template <int N, typename T, bool HELM, bool FUSEP, bool AFF>
+static cudaError_t launch_ax_a(cudaStream_t s, int nel, int epb, T* u, T* au, const T* gf,
                                size_t npts, const double* bj, const double* D,
                                const double* S, double lambda, const PUpdate& pu,
-                               const ScalarOp& dop) {
+                               const ScalarOp& dop, const AffGeom& ag) {
+  if (epb == kAxLine) {
+    using L = AxLine<N>;
+    constexpr size_t smem = (size_t)L::SMEM * sizeof(T);
+    static SmemAttr attr;
+    cudaError_t e = attr.ensure((const void*)k_axl<N, T, HELM, FUSEP, AFF>, smem);
+    if (e != cudaSuccess) return e;
+    const int grd = (nel + L::EPB - 1) / L::EPB;
+    SSG_COUNT();
+    k_axl<N, T, HELM, FUSEP, AFF><<<grd, L::THREADS, smem, s>>>(nel, u, au, gf, npts, bj, D, S,
+                                                               lambda, pu, dop, ag);
+    return cudaGetLastError();
+  }
   const size_t smem = (4 * N * AxLayout<N>::P + (size_t)epb * 3 * N * N * AxLayout<N>::Q) *
                       sizeof(double);
   static SmemAttr attr;
-  {
-    cudaError_t e = attr.ensure((const void*)k_ax<N, T, HELM, FUSEP>, 200 * 1024);
-    if (e != cudaSuccess) return e;
-  }
+  cudaError_t e = attr.ensure((const void*)k_ax<N, T, HELM, FUSEP, AFF>, 200 * 1024);
+  if (e != cudaSuccess) return e;
   dim3 blk(N, N, epb);
   dim3 grd((nel + epb - 1) / epb);
-  { SSG_COUNT(); k_ax<N, T, HELM, FUSEP><<<grd, blk, smem, s>>>(nel, u, au, gf, npts, bj, D, S, lambda, pu, dop); }
-  return cudaGetLastError();
-}
-
-template <int N, typename T, bool HELM, bool FUSEP>
-static cudaError_t launch_axl_t(cudaStream_t s, int nel, T* u, T* au, const T* gf,
-                                size_t npts, const double* bj, const double* D,
-                                const double* S, double lambda, const PUpdate& pu,
-                                const ScalarOp& dop) {
-  using L = AxLine<N>;
-  constexpr size_t smem = (size_t)L::SMEM * sizeof(T);
-  static SmemAttr attr;
-  {
-    cudaError_t e = attr.ensure((const void*)k_axl<N, T, HELM, FUSEP>, smem);
-    if (e != cudaSuccess) return e;
-  }
-  const int grd = (nel + L::EPB - 1) / L::EPB;
-  { SSG_COUNT(); k_axl<N, T, HELM, FUSEP><<<grd, L::THREADS, smem, s>>>(nel, u, au, gf, npts, bj, D, S, lambda, pu, dop); }
+  SSG_COUNT();
+  k_ax<N, T, HELM, FUSEP, AFF><<<grd, blk, smem, s>>>(nel, u, au, gf, npts, bj, D, S, lambda, pu,
+                                                     dop, ag);
   return cudaGetLastError();
 }
 
@@ -974,15 +972,14 @@ template <typename T, bool HELM, bool FUSEP>
 static cudaError_t ax_dispatch(int n, cudaStream_t s, int nel, int epb, T* u, T* au,
                                const T* gf, size_t npts, const double* bj, const double* D,
                                const double* S, double lambda, const PUpdate& pu,
-                               const ScalarOp& dop) {
+                               const ScalarOp& dop, const AffGeom& ag) {
   switch (n) {
-#define SSG_AXN(NV)                                                                   \
-  case NV:                                                                            \
-    if (epb == kAxLine)                                                               \
-      return launch_axl_t<NV, T, HELM, FUSEP>(s, nel, u, au, gf, npts, bj, D, S,      \
-                                              lambda, pu, dop);                       \
-    return launch_ax_t<NV, T, HELM, FUSEP>(s, nel, epb, u, au, gf, npts, bj, D, S,    \
-                                           lambda, pu, dop);
+#define SSG_AXN(NV)                                                                         \
+  case NV:                                                                                  \
+    return ag.c ? launch_ax_a<NV, T, HELM, FUSEP, true>(s, nel, epb, u, au, gf, npts, bj, D, \
+                                                        S, lambda, pu, dop, ag)             \
+                : launch_ax_a<NV, T, HELM, FUSEP, false>(s, nel, epb, u, au, gf, npts, bj,  \
+                                                         D, S, lambda, pu, dop, ag);
     SSG_AXN(2) SSG_AXN(3) SSG_AXN(4) SSG_AXN(5) SSG_AXN(6) SSG_AXN(7)
     SSG_AXN(8) SSG_AXN(9) SSG_AXN(10) SSG_AXN(11) SSG_AXN(12)
 #undef SSG_AXN
@@ -993,7 +990,7 @@ static cudaError_t ax_dispatch(int n, cudaStream_t s, int nel, int epb, T* u, T*
 cudaError_t run_ax(cudaStream_t s, int n, int nel, int epb, bool helm, bool fp32,
                    const void* in, void* out, const void* gf, size_t npts,
                    const double* bj, const double* D, const double* S, double lambda,
-                   const PUpdateArgs* pua) {
+                   const PUpdateArgs* pua, const AffGeom& ag) {
   PUpdate pu;
   const bool fuse = pua != nullptr;
   ScalarOp dop;
@@ -1016,28 +1013,28 @@ cudaError_t run_ax(cudaStream_t s, int n, int nel, int epb, bool helm, bool fp32
   const bool dmma = n == 8 && !fp32;
   if (dmma)
     return run_ax8_dmma(s, nel, helm, fp32, (void*)in, out, gf, npts, bj, D, S, lambda,
-                        fuse ? &pu : nullptr, &dop);
+                        fuse ? &pu : nullptr, &dop, ag);
   if (epb == 0) epb = ax_epb(n);
   if (fp32) {
     if (helm) return cudaErrorInvalidValue;
     if (fuse)
       return ax_dispatch<float, false, true>(n, s, nel, epb, (float*)in, (float*)out,
-                                             (const float*)gf, npts, nullptr, D, D, 0.0, pu, dop);
+                                             (const float*)gf, npts, nullptr, D, D, 0.0, pu, dop, ag);
     return ax_dispatch<float, false, false>(n, s, nel, epb, (float*)in, (float*)out,
-                                            (const float*)gf, npts, nullptr, D, D, 0.0, pu, dop);
+                                            (const float*)gf, npts, nullptr, D, D, 0.0, pu, dop, ag);
   }
   if (helm) {
     if (fuse)
       return ax_dispatch<double, true, true>(n, s, nel, epb, (double*)in, (double*)out,
-                                             (const double*)gf, npts, bj, D, S, lambda, pu, dop);
+                                             (const double*)gf, npts, bj, D, S, lambda, pu, dop, ag);
     return ax_dispatch<double, true, false>(n, s, nel, epb, (double*)in, (double*)out,
-                                            (const double*)gf, npts, bj, D, S, lambda, pu, dop);
+                                            (const double*)gf, npts, bj, D, S, lambda, pu, dop, ag);
   }
   if (fuse)
     return ax_dispatch<double, false, true>(n, s, nel, epb, (double*)in, (double*)out,
-                                            (const double*)gf, npts, nullptr, D, D, 0.0, pu, dop);
+                                            (const double*)gf, npts, nullptr, D, D, 0.0, pu, dop, ag);
   return ax_dispatch<double, false, false>(n, s, nel, epb, (double*)in, (double*)out,
-                                           (const double*)gf, npts, nullptr, D, D, 0.0, pu, dop);
+                                           (const double*)gf, npts, nullptr, D, D, 0.0, pu, dop, ag);
 }
 
 // one 256-thread block per 256 node tasks, capped at bps blocks per SM

@@ -455,14 +455,15 @@ __device__ __forceinline__ void ax_load_mats(double* sD, const double* __restric
 // false for a padding slot).  Returns this thread's share of p . (A p)
 // (FUSEP).  sD: the four matrices (ax_load_mats); su, sw0, sw1: this
 // slot's planes.
-template <int N, typename T, bool HELM, bool FUSEP>
+template <int N, typename T, bool HELM, bool FUSEP, bool AFF = false>
 __device__ __forceinline__ double ax_element(int e, bool active, int i, int j, const double* sD,
                                              double* su, double* sw0, double* sw1,
                                              T* __restrict__ u, T* __restrict__ au,
                                              const T* __restrict__ gf, size_t npts,
                                              const double* __restrict__ bj, double lambda,
                                              const T* __restrict__ z, double beta, double c,
-                                             const double* __restrict__ mask, bool first) {
+                                             const double* __restrict__ mask, bool first,
+                                             const AffGeom& ag = AffGeom()) {
   constexpr int NN = N * N, P = AxSmem<N>::P, Q = AxSmem<N>::Q, PLANE = AxSmem<N>::PLANE;
   const double* sDT = sD + N * P;
   const double* sS = sDT + N * P;
@@ -495,6 +496,13 @@ __device__ __forceinline__ double ax_element(int e, bool active, int i, int j, c
   __syncthreads();
   // r-derivative with S for Helmholtz (the swapped deriv_matrix), D otherwise
   const double* Dx = HELM ? sS : sD;
+  // affine: the element's constant metric, the weights of this column
+  double cg[6], wij = 0.0;
+  if (AFF) {
+#pragma unroll
+    for (int a = 0; a < 6; ++a) cg[a] = active ? __ldg(ag.c + 6 * (size_t)e + a) : 0.0;
+    wij = __ldg(ag.w + i) * __ldg(ag.w + j);
+  }
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     const double ur = row_dot<N>(Dx + i * P, su + k * PLANE + j * Q);
@@ -502,7 +510,11 @@ __device__ __forceinline__ double ax_element(int e, bool active, int i, int j, c
     const double ut = row_reg_dot<N>(sD + k * P, ru);
     const size_t o = off + (size_t)k * NN;
     double g0 = 0, g1 = 0, g2 = 0, g3 = 0, g4 = 0, g5 = 0;
-    if (active) {
+    if (AFF) {
+      const double rho = wij * __ldg(ag.w + k);
+      g0 = cg[0] * rho; g1 = cg[1] * rho; g2 = cg[2] * rho;
+      g3 = cg[3] * rho; g4 = cg[4] * rho; g5 = cg[5] * rho;
+    } else if (active) {
       g0 = (double)__ldg(gf + o);
       g1 = (double)__ldg(gf + npts + o);
       g2 = (double)__ldg(gf + 2 * npts + o);
@@ -545,7 +557,10 @@ __device__ __forceinline__ double ax_element(int e, bool active, int i, int j, c
 // reads the same entry (a broadcast), two entries per paired load.  EPB
 // elements per group fill about 256 threads.  The arithmetic runs in the
 // storage type T: FP64 for the solves, FP32 in the mixed-precision V-cycle
-// (the fused direction update and the p . (A p) sum stay FP64).
+// (the fused direction update and the p . (A p) sum stay FP64).  AFF: a
+// level of affine elements reads six constants an element instead of six
+// factors a point (Helmholtz at n = 12 on 576 elements, fused: 36.7 us with
+// the factors, 26.2 without; FP32 at n = 8 on 4096: 34.1 and 25.0).
 // ---------------------------------------------------------------------------
 template <int N>
 struct AxLine {
@@ -615,7 +630,7 @@ __device__ __forceinline__ void axl_load_mats(T* sD, const double* __restrict__ 
 // p = (first ? z - c : beta u + (z - c)) .* mask, written back to u.
 // rdot, mult (optional): also sum (rdot w) p over the staged points, w =
 // 1 / mult, into *rdz.  Returns this thread's share of p . (A p) (FUSEP).
-template <int N, typename T, bool HELM, bool FUSEP>
+template <int N, typename T, bool HELM, bool FUSEP, bool AFF>
 __device__ __forceinline__ double axl_group(int e0, int ne, T* __restrict__ u,
                                             T* __restrict__ au, const T* __restrict__ gf,
                                             size_t npts, const double* __restrict__ bj,
@@ -623,7 +638,8 @@ __device__ __forceinline__ double axl_group(int e0, int ne, T* __restrict__ u,
                                             double beta, double c,
                                             const double* __restrict__ mask, bool first,
                                             T* sD, const T* __restrict__ rdot,
-                                            const uint8_t* __restrict__ mult, double* rdz) {
+                                            const uint8_t* __restrict__ mult, double* rdz,
+                                            const AffGeom& ag) {
   using L = AxLine<N>;
   using C = T;
   constexpr int NN = N * N, NT = N * N * N, RM = L::RM, RS = L::RS, FS = L::FS;
@@ -637,7 +653,7 @@ __device__ __forceinline__ double axl_group(int e0, int ne, T* __restrict__ u,
   // the group's six metric chunks into L2 now: they are read only after
   // the three derivative passes (a hint, no buffer; 16-byte aligned chunks
   // of a multiple of 16 bytes only)
-  if (tid < 6 && npb > 0) {
+  if (!AFF && tid < 6 && npb > 0) {
     const T* chunk = gf + (size_t)tid * npts + base;
     const unsigned bytes = (unsigned)(npb * sizeof(T));
     if (((reinterpret_cast<uintptr_t>(chunk) | bytes) & 15u) == 0)
@@ -696,15 +712,33 @@ __device__ __forceinline__ double axl_group(int e0, int ne, T* __restrict__ u,
     const C* src = U + a1 * RS + a0;
 #pragma unroll
     for (int l = 0; l < N; ++l) x[l] = src[l * N * RS];
+    // affine: the element's constant metric, the weights of this line
+    C cg[6];
+    double wij = 0.0;
+    if (AFF) {
+#pragma unroll
+      for (int a = 0; a < 6; ++a) cg[a] = (C)__ldg(ag.c + 6 * (size_t)(e0 + sl) + a);
+      wij = __ldg(ag.w + a0) * __ldg(ag.w + a1);
+    }
 #pragma unroll 2
     for (int k = 0; k < N; ++k) {
       const C ut = line_row<N, RM, C>(sD, k, x);
       const int q = k * N * RS + a1 * RS + a0;
       const size_t o = eo + (size_t)k * NN;
       const C ur = F1[q], us = F2[q];
-      const C g0 = __ldg(gf + o), g1 = __ldg(gf + npts + o), g2 = __ldg(gf + 2 * npts + o),
-              g3 = __ldg(gf + 3 * npts + o), g4 = __ldg(gf + 4 * npts + o),
-              g5 = __ldg(gf + 5 * npts + o);
+      C g0, g1, g2, g3, g4, g5;
+      if (AFF) {
+        const C rho = (C)(wij * __ldg(ag.w + k));
+        g0 = cg[0] * rho; g1 = cg[1] * rho; g2 = cg[2] * rho;
+        g3 = cg[3] * rho; g4 = cg[4] * rho; g5 = cg[5] * rho;
+      } else {
+        g0 = __ldg(gf + o);
+        g1 = __ldg(gf + npts + o);
+        g2 = __ldg(gf + 2 * npts + o);
+        g3 = __ldg(gf + 3 * npts + o);
+        g4 = __ldg(gf + 4 * npts + o);
+        g5 = __ldg(gf + 5 * npts + o);
+      }
       F1[q] = g0 * ur + g1 * us + g2 * ut;
       F2[q] = g1 * ur + g3 * us + g4 * ut;
       w2[k] = g2 * ur + g4 * us + g5 * ut;

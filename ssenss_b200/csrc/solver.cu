@@ -240,7 +240,7 @@ ssg_status op_apply(ssg_context* c, int level, int var, bool fp32, const void* i
   void* loc = global ? (fp32 ? c->ws->w32[level].aploc : c->ws->w64[level].aploc) : out;
   SSG_CUDA(c, run_ax(c->stream, L.n, c->nel, 0, helm, fp32, in, loc,
                      fp32 ? (const void*)L.gf32 : (const void*)L.gf, L.npts, L.bj, L.D, L.S,
-                     lambda_of(c), nullptr));
+                     lambda_of(c), nullptr, aff_geom(L)));
   if (global)
     SSG_CUDA(c, run_dss(c->stream, DSS_PLAIN, fp32, L.n, c->nel, loc, out, c->d_nbreg, L.dss_ec,
                         helm ? L.mask : nullptr, nullptr, nullptr, nullptr));
@@ -302,7 +302,7 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
   // mask f; r = f - A x; subtract_nullspace(r)
   if (mask) SSG_CUDA(c, run_mul(s, fp32, np, f, mask));
   SSG_CUDA(c, run_ax(s, L.n, c->nel, 0, helm, fp32, x, W.aploc, gf, np, L.bj, L.D, L.S, lam,
-                     nullptr));
+                     nullptr, aff_geom(L)));
   op.code = OP_NULL_C;
   SSG_CUDA(c, run_dss(s, DSS_RESID, fp32, L.n, c->nel, W.aploc, W.r, c->d_nbreg, L.dss_ec, mask, f,
                       nullptr, c->d_part, nullptr, &op));
@@ -381,7 +381,7 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
             c, true, stop,
             [&]() -> ssg_status {
               SSG_CUDA(c, run_ax(s, L.n, c->nel, 0, helm, fp32, W.p, W.aploc, gf, np, L.bj, L.D,
-                                 L.S, lam, &pu));
+                                 L.S, lam, &pu, aff_geom(L)));
               if (fused) {
                 op.code = OP_CG_BETA;
                 SSG_CUDA(c, run_dss(s, DSS_CGUPD, fp32, L.n, c->nel, W.aploc, nullptr, c->d_nbreg,
@@ -422,7 +422,7 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
     pu.first = it == 0;
     dop.code = it == 0 ? OP_STORE_PAP : OP_CG_ALPHA;
     SSG_CUDA(c, run_ax(s, L.n, c->nel, 0, helm, fp32, W.p, W.aploc, gf, np, L.bj, L.D, L.S,
-                       lam, &pu));
+                       lam, &pu, aff_geom(L)));
     if (it == 0) {
       // rdz = (r w).p, |r|_w (src/solver.c:58-61) (fused: and alpha)
       PtrList ys;
@@ -506,7 +506,7 @@ static ssg_status mg_recurse(ssg_context* c, int L, void* f, void* x, double eps
     // r = f - A x (compute_residual, src/precon.c:302-309)
     SSG_CUDA(c, run_ax(s, F.n, c->nel, 0, false, fp32, x, W.aploc,
                        fp32 ? (const void*)F.gf32 : (const void*)F.gf, F.npts, nullptr, F.D,
-                       F.D, 0.0, nullptr));
+                       F.D, 0.0, nullptr, aff_geom(F)));
     SSG_CUDA(c, run_dss(s, DSS_RESID, fp32, F.n, c->nel, W.aploc, W.rr, c->d_nbreg, F.dss_ec, nullptr,
                         f, nullptr, c->d_part));
     rin = W.rr;
@@ -655,7 +655,7 @@ ssg_status fcg_solve(ssg_context* c, const double* f, double* u, double eps, int
 
   // r = f - A u; subtract_nullspace(r)
   SSG_CUDA(c, run_ax(s, L.n, c->nel, 0, false, false, u, w->aploc, L.gf, np, nullptr, L.D,
-                     L.D, 0.0, nullptr));
+                     L.D, 0.0, nullptr, aff_geom(L)));
   op.code = OP_NULL_C;
   SSG_CUDA(c, run_dss(s, DSS_RESID, false, L.n, c->nel, w->aploc, w->r, c->d_nbreg, L.dss_ec, nullptr,
                       f, nullptr, c->d_part, nullptr, &op));
@@ -720,7 +720,7 @@ ssg_status fcg_solve(ssg_context* c, const double* f, double* u, double eps, int
     double* ap0 = w->AP[aslot[0]];
     // ap0 = A p0; pap0 and alpha = (p0 w).r / pap0
     SSG_CUDA(c, run_ax(s, L.n, c->nel, 0, false, false, p0, w->aploc, L.gf, np, nullptr, L.D,
-                       L.D, 0.0, nullptr));
+                       L.D, 0.0, nullptr, aff_geom(L)));
     op.pap_idx[0] = aslot[0];
     op.code = OP_FCG_ALPHA;
     SSG_CUDA(c, run_dss(s, DSS_DOT2, false, L.n, c->nel, w->aploc, ap0, c->d_nbreg, L.dss_ec, nullptr,

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "ssenss_b200.h"
+#include "ssg_kernels.h"
 
 #define SSG_MAXLEV 8
 #define SSG_MAXN 18
@@ -86,6 +87,9 @@ ssg_status build_mesh(HostMesh& m, int n, int nel, const double* vertices,
                       const int* neigh, std::string& err, unsigned opts = 0,
                       int svvn = -1, double svva = 0.0);
 ssg_status build_pairs(HostMesh& m, std::string& err, bool opposite = false);
+// The constant metric of each element (nel x 6: G_ab J) where every element
+// of the level is an affine image of the reference cube; empty otherwise.
+void affine_metric(const HostLevel& L, int nel, std::vector<double>& c);
 void stiffness_diagonal(const HostLevel& L, int nel, double* out);
 void host_dss(const HostMesh& m, int n, double* u);
 // DSS map of one level (one int array):
@@ -109,6 +113,8 @@ struct DevLevel {
   size_t nt = 0, npts = 0;
   double* gf = nullptr;        // 6 x npts: G_ab * rho * J
   double* bj = nullptr;        // rho * J
+  double* aff = nullptr;       // nel x 6: G_ab J where every element is affine, else null
+  double* w = nullptr;         // n GLL weights (with aff)
   double* kdiag = nullptr;     // element-local stiffness diagonal
   double* dinv_p = nullptr;    // Poisson Jacobi inverse
   double* dinv_h = nullptr;    // Helmholtz Jacobi inverse (for lambda_h)
@@ -126,6 +132,13 @@ struct DevLevel {
   double nunique = 0.0;        // sum of 1/multiplicity
   double lambda_h = -1.0;      // lambda the Helmholtz diagonal holds
 };
+
+inline AffGeom aff_geom(const DevLevel& L) {
+  AffGeom a;
+  a.c = L.aff;
+  a.w = L.w;
+  return a;
+}
 
 struct Workspace;
 

@@ -84,6 +84,17 @@ struct PUpdateArgs {
   double* part = nullptr;
 };
 
+// Geometry of a level whose every element is an affine image of the
+// reference cube (DevLevel::aff): the metric of element e is constant,
+// G_ab det J = c[6 e + ab] (order 11, 12, 13, 22, 23, 33), and the factor
+// at a node is that constant times the node's weight product w_i w_j w_k.
+// The operator then reads six values an element instead of six a point.
+// c == nullptr: use the per-point factors.
+struct AffGeom {
+  const double* c = nullptr;
+  const double* w = nullptr;   // n GLL weights
+};
+
 // kernel launches of this library: process-wide, and per host thread (the
 // per-thread count tells a stream capture how many launches it recorded)
 extern std::atomic<unsigned long long> g_launches;
@@ -137,12 +148,12 @@ namespace dev { struct PUpdate; }
 cudaError_t run_ax8_dmma(cudaStream_t s, int nel, bool helm, bool fp32, void* u, void* au,
                          const void* gf, size_t npts, const double* bj, const double* D,
                          const double* S, double lambda, const dev::PUpdate* pu,
-                         const ScalarOp* dop);
+                         const ScalarOp* dop, const AffGeom& ag);
 
 cudaError_t run_ax(cudaStream_t s, int n, int nel, int epb, bool helm, bool fp32,
                    const void* in, void* out, const void* gf, size_t npts,
                    const double* bj, const double* D, const double* S, double lambda,
-                   const PUpdateArgs* pua);
+                   const PUpdateArgs* pua, const AffGeom& ag = AffGeom());
 // ints before the edge/corner records of a DSS map: one gather word per
 // local point, rounded up to 16 bytes
 inline __host__ __device__ constexpr size_t dss_map_records_offset(size_t npts) {

@@ -58,11 +58,11 @@ static ssg_status tune_level(ssg_context* c, int level, double* a, double* b, do
     for (int epb = kAxLine; epb <= ax_epb_max(n); epb = epb == kAxLine ? 1 : 2 * epb) {
       g_tune_ax_epb[n] = epb;
       SSG_CUDA(c, run_ax(c->stream, n, c->nel, epb, false, false, a, b, L.gf, L.npts, nullptr,
-                         L.D, L.D, 0.0, nullptr));
+                         L.D, L.D, 0.0, nullptr, aff_geom(L)));
       float t = 0.f;
       SSG_TRY(time_launches(c, reps, [&] {
         return run_ax(c->stream, n, c->nel, epb, false, false, a, b, L.gf, L.npts, nullptr,
-                      L.D, L.D, 0.0, nullptr);
+                      L.D, L.D, 0.0, nullptr, aff_geom(L));
       }, &t));
       if (t < best) {
         best = t;
@@ -180,7 +180,7 @@ ssg_status ssg_time_operator(ssg_context* c, int var, int reps, double* us_per_a
   SSG_TRY(fill_field(c, in, L.npts));
   auto launch = [&] {
     return run_ax(c->stream, L.n, c->nel, 0, helm, false, in, out, L.gf, L.npts, L.bj, L.D,
-                  L.S, lam, nullptr);
+                  L.S, lam, nullptr, aff_geom(L));
   };
   SSG_CUDA(c, launch());
   float best = 0.f;
@@ -215,7 +215,7 @@ ssg_status ssg_time_smoother(ssg_context* c, int level, int reps, double* us) {
   const int nb = vec_blocks(np);
   auto op = [&] {
     return run_ax(c->stream, L.n, c->nel, 0, false, false, buf[0], buf[1], L.gf, np, nullptr,
-                  L.D, L.D, 0.0, nullptr);
+                  L.D, L.D, 0.0, nullptr, aff_geom(L));
   };
   auto dss = [&] {
     return run_dss(c->stream, DSS_DOT, false, L.n, c->nel, buf[1], buf[2], c->d_nbreg,
