@@ -67,6 +67,13 @@ static void free_level(ssg::DevLevel& d) {
   d = ssg::DevLevel();
 }
 
+static void free_conv(ssg_context* c) {
+  dfree(c->conv_w); dfree(c->conv_D); dfree(c->conv_J);
+  dfree(c->conv_scratch); dfree(c->conv_aff);
+  c->conv_w = c->conv_D = c->conv_J = c->conv_scratch = c->conv_aff = nullptr;
+  for (auto& v : c->conv_eo) v.clear();
+}
+
 static void free_mesh(ssg_context* c) {
   c->dev_bytes = 0;
   if (c->ws) {
@@ -93,9 +100,7 @@ static void free_mesh(ssg_context* c) {
   dfree(c->d_pairs); c->d_pairs = nullptr;
   dfree(c->d_nbreg); c->d_nbreg = nullptr;
   dfree(c->inv_mass); c->inv_mass = nullptr;
-  dfree(c->conv_w); dfree(c->conv_D); dfree(c->conv_J);
-  dfree(c->conv_scratch);
-  c->conv_w = c->conv_D = c->conv_J = c->conv_scratch = nullptr;
+  free_conv(c);
   c->m = 0;
   dfree(c->p_jac); dfree(c->p_tinv); dfree(c->p_ur); dfree(c->p_x);
   c->p_jac = c->p_tinv = c->p_ur = c->p_x = nullptr;
@@ -134,9 +139,7 @@ static ssg_status upload_conv(ssg_context* c) {
   const ssg::HostMesh& H = c->host;
   const ssg::HostLevel& m = H.conv;
   const int nel = H.nel;
-  dfree(c->conv_w); dfree(c->conv_D); dfree(c->conv_J);
-  dfree(c->conv_scratch);
-  c->conv_w = c->conv_D = c->conv_J = c->conv_scratch = nullptr;
+  free_conv(c);
   c->m = m.n;
   const size_t mp = m.nt * nel;
   const std::vector<double> rho = rho3(m.w);
@@ -145,15 +148,30 @@ static ssg_status upload_conv(ssg_context* c) {
     for (int a = 0; a < 3; ++a) {
       const double* t = m.tinv[3 * a + b].data();
       double* dst = wv.data() + (size_t)(3 * b + a) * mp;
-      for (int e = 0; e < nel; ++e)
-        for (size_t q = 0; q < m.nt; ++q) {
-          const size_t g = e * m.nt + q;
-          dst[g] = 0.5 * ((rho[q] * m.det[g]) * t[g]);
-        }
+      parallel_elements(nel, [&](int e0, int e1) {
+        for (int e = e0; e < e1; ++e)
+          for (size_t q = 0; q < m.nt; ++q) {
+            const size_t g = e * m.nt + q;
+            dst[g] = 0.5 * ((rho[q] * m.det[g]) * t[g]);
+          }
+      });
     }
   SSG_TRY(dupload(c, &c->conv_w, wv.data(), wv.size()));
   SSG_TRY(dupload(c, &c->conv_D, m.D.data(), m.D.size()));
   SSG_TRY(dupload(c, &c->conv_J, H.jconv.data(), H.jconv.size()));
+  std::vector<double> aff;
+  affine_convection(m, nel, aff);
+  // (the affine form folds the quadrature weights into the projection)
+  std::vector<double> P((size_t)H.n * m.n);
+  for (int p = 0; p < H.n; ++p)
+    for (int o = 0; o < m.n; ++o)
+      P[(size_t)p * m.n + o] = H.jconv[(size_t)o * H.n + p] * (aff.empty() ? 1.0 : m.w[o]);
+  std::vector<double>* eo = c->conv_eo;
+  if (!conv_eo_split(H.n, m.n, H.jconv.data(), false, eo[0], eo[1]) ||
+      !conv_eo_split(m.n, m.n, m.D.data(), true, eo[2], eo[3]) ||
+      !conv_eo_split(m.n, H.n, P.data(), false, eo[4], eo[5]))
+    for (int k = 0; k < 6; ++k) eo[k].clear();
+  if (!aff.empty() && !eo[0].empty()) SSG_TRY(dupload(c, &c->conv_aff, aff.data(), aff.size()));
   const size_t scr = convection_scratch_doubles(H.n, m.n);
   if (scr) SSG_TRY(dalloc(c, &c->conv_scratch, scr));
   return SSG_OK;
@@ -941,8 +959,7 @@ ssg_status ssg_convection_operator(ssg_context* c, const double* u, const double
     SSG_TRY(stage_in(c, 1, v, np, &dv));
   SSG_TRY(stage_out(c, 2, udv, np, &dout));
   SSG_CUDA(c, run_convection(c->stream, c->nel, 0, c->nel, c->n, c->m, du, dv, dout,
-                             c->conv_w, c->host.conv.D.data(), c->host.jconv.data(),
-                             c->conv_D, c->conv_J, c->conv_scratch));
+                             conv_geom(c)));
   return stage_back(c, udv, dout, np);
 }
 
@@ -963,8 +980,7 @@ ssg_status ssg_convection_elements(ssg_context* c, int first, int count, const d
     SSG_TRY(stage_in(c, 1, v, np, &dv));
   SSG_TRY(stage_out(c, 2, udv, np, &dout));
   SSG_CUDA(c, run_convection(c->stream, count, first, c->nel, c->n, c->m, du, dv, dout,
-                             c->conv_w, c->host.conv.D.data(), c->host.jconv.data(),
-                             c->conv_D, c->conv_J, c->conv_scratch));
+                             conv_geom(c)));
   return stage_back(c, udv, dout, np);
 }
 

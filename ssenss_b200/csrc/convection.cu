@@ -1,6 +1,5 @@
 // Dealiased skew-symmetric convection (convection_operator ->
-// antialiased_convection_operator, src/convection.c:31-140), one element per
-// block, all in FP64:
+// antialiased_convection_operator, src/convection.c:31-140), all in FP64:
 //   1. interpolate the advecting u and advected v (3 components each) from
 //      the n-point to the m = 3n/2-point GLL grid (interpolate_to_grid,
 //      src/interpolation.c:136-155);
@@ -15,24 +14,38 @@
 // Step 2 is regrouped per reference direction b (the same sums):
 //   skew = sum_b ( A_b d_b v_c + B_b d_b(u_b v_c) ),
 //   A_b = sum_a u_a W[a][b],  B_b = sum_a W[a][b],  W[a][b] = rho J tinv[a][b] / 2,
-// with W stored at set-up.  So each direction b is one pass over the
-// m-point lines along b: a thread holds one line of v_c and of u_b v_c in
-// registers, takes both derivatives along it and adds its points' A_b and
-// B_b terms -- the contributions of the three directions meet in shared
-// memory.  Every contraction (interpolation, derivative, projection) works
-// on whole lines held in registers, and the small matrices (D, J, J^T) live
-// in the kernel's parameter space: with the loops unrolled, each matrix
-// entry is a constant-bank operand of the FMA, so the shared-memory pipe
-// carries only the line loads (one per line point instead of two per FMA).
+// so each direction b is one pass over the m-point lines along b.
 //
-// Orders with m^3 fields beyond shared memory (n = 12) and dealiasing orders
-// other than 3n/2 run a runtime-order kernel of the same arithmetic that
-// keeps the matrices in shared memory and its fields in a global scratch
-// region when needed.
+// k_conv_line (m = 3n/2, n <= 12): what bounds it is the FP64 pipe and the
+// shared-memory pipe together, so it is built to spend few of either.
+//  - Every contraction (interpolation, derivative, projection) is one whole
+//    line in one thread's registers: a line is loaded once for all its
+//    outputs, and the small matrices sit in the kernel's parameter space, so
+//    an entry is a constant-bank operand of the FMA.
+//  - The GLL points are symmetric about 0, so the matrices are too
+//    (J[M-1-o][N-1-p] = J[o][p], D[M-1-i][M-1-l] = -D[i][l]): a line is
+//    split into its even and odd parts, each contracted with a matrix of a
+//    quarter of the entries -- half the multiply-adds.  (The FP64 tensor
+//    cores have the same peak as the FMA pipe, and their 8 x 8 x 4 tiles pad
+//    m = 12 to 16 columns: the same work there is 2.6 times as many
+//    operations.)
+//  - Stages run in place: a thread overwrites the line it read, so the only
+//    buffers are the fields themselves (U, V, SK) and all components of a
+//    stage go through one sweep between two barriers.
+//  - On affine elements (constant metric) the weights W reduce to nine
+//    numbers an element, and the quadrature weights fold into the projection
+//    matrix: no weight is read per point.
+//
+// Matrices without that symmetry (a caller's own arrays), dealiasing orders
+// other than 3n/2 and fields at addresses that are not 16-byte aligned run a
+// runtime-order kernel of the same arithmetic.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
+#include <iterator>
+#include <type_traits>
 #include <vector>
 
 #include "kernels.cuh"
@@ -46,46 +59,88 @@ namespace dev {
 // compile-time-order kernel
 // ----------------------------------------------------------------------------
 
-// row stride of an m-wide shared array: 2 mod 4 doubles, so that the
-// 16-byte loads of lines along i by lanes walking j hit distinct banks
-__host__ __device__ constexpr int conv_row(int w) { return w + ((2 - w % 4) + 4) % 4; }
+// row stride of the m-wide shared fields: odd for odd m (scalar accesses),
+// 2 mod 4 doubles for even m (16-byte accesses along i), so that lanes
+// walking j hit distinct banks
+__host__ __device__ constexpr int conv_row(int m) { return m % 2 ? m : (m % 4 == 2 ? m : m + 2); }
 
+// A matrix entry in the kernel's parameter space, padded to 16 bytes: next
+// to each other the compiler loads entries in pairs into registers, keeps
+// them there across the line loop and spills (n = 8: 377 us a call on 4096
+// elements); apart, each is a constant operand of its multiply-add
+struct ConvEntry {
+  double v, pad;
+};
+
+// even / odd halves of the three matrices (h = number of even terms)
 template <int N, int M>
 struct ConvMats {
-  double D[M * M];   // D[o * M + l] = l_l'(x_o), m-point grid
-  double J[M * N];   // J[o * N + p] = l_p^n(x_o^m)
-  double JT[N * M];  // JT[p * M + o] = J[o * N + p]
+  static constexpr int HN = (N + 1) / 2, HM = (M + 1) / 2;
+  ConvEntry JE[HM * HN], JO[HM * HN];   // interpolation n -> m
+  ConvEntry DE[HM * HM], DO[HM * HM];   // derivative on m points
+  ConvEntry PE[HN * HM], PO[HN * HM];   // projection m -> n (weights folded in when affine)
 };
 
-template <int N, int M>
-struct ConvLayout {
-  static constexpr int RM = conv_row(M);      // row stride, m-wide rows
-  static constexpr int RN = conv_row(N);      // row stride, n-wide rows
-  static constexpr int FM = M * M * RM;       // an m^3 field
-  static constexpr int T1 = N * N * RM;       // interpolation stage x: [k][j][o]
-  static constexpr int T2 = N * M * RM;       // stage y: [k][o2][o1]
-  static constexpr int P1 = M * M * RN;       // projection stage i: [k][j][p]
-  static constexpr int P2 = M * N * RN;       // stage j: [k][p2][p1]
-  // UI (3 FM), VC (FM), SK (FM), T1, T2; P1 reuses VC, P2 reuses T2
-  static constexpr int TOTAL = 5 * FM + T1 + T2;
-  static_assert(P1 <= FM && P2 <= T2, "projection scratch aliases");
+template <int N>
+struct ConvLine {
+  static constexpr int M = (3 * N) / 2;
+  static constexpr int RM = conv_row(M), PL = M * RM, FM = M * PL;
+  // components advected together: three while the nine fields fit
+  static constexpr int NB = (size_t)9 * FM * 8 <= 200 * 1024 ? 3 : 1;
+  // n = 12: U, V and SK together exceed a block's shared memory by 832
+  // bytes, so SK (written and read once a pass) lives in the block's part of
+  // the global scratch and stays in L2
+  static constexpr bool GSK = (size_t)(3 + 2 * NB) * FM * 8 > 227 * 1024;
+  // per-point weights: A_b and B_b of the direction at hand as two more
+  // fields, formed point by point with coalesced weight loads, once for all
+  // components (lines reading the weights themselves: 143.6 us a call at
+  // n = 8 on 1024 deformed elements); n >= 11 has no room for them
+  static constexpr bool AB = (size_t)(5 + 2 * NB) * FM * 8 <= 227 * 1024;
+  static constexpr size_t smem(bool aff) {
+    return (size_t)(3 + (GSK ? 1 : 2) * NB + (!aff && AB ? 2 : 0)) * FM * sizeof(double);
+  }
+  static constexpr int TASKS = NB * M * M;
+  // one line a thread, 128 registers at 512 threads; 448 threads (m = 12)
+  // put four warps on two of the SM's four schedulers, so they would have the
+  // registers of 512: 384 threads have 168 and the same longest scheduler
+  static constexpr int FULL = (TASKS + 31) / 32 * 32;
+  static constexpr int THREADS = N == 12 ? 256 : (FULL > 384 && FULL < 512 ? 384 : FULL);
+  // small orders: several blocks per SM
+  static constexpr int BLOCKS = THREADS <= 128 ? 4 : (THREADS <= 256 && NB == 3 ? 2 : 1);
 };
 
-template <int N, int M>
-constexpr size_t conv_smem_bytes() {
-  return (size_t)ConvLayout<N, M>::TOTAL * sizeof(double);
-}
-
-// y[o] = sum_{l < NI} A[o * NI + l] x[l], summed in l order
-template <int NI, int NO>
-__device__ __forceinline__ void line_contract(const double* A, const double (&x)[NI],
-                                              double (&y)[NO]) {
+// y (NO) = A x (NI), A symmetric under reversal of both indices (ANTI:
+// antisymmetric), as its even / odd halves E, O
+template <int NI, int NO, bool ANTI>
+__device__ __forceinline__ void eo_contract(const ConvEntry* E, const ConvEntry* O,
+                                            const double (&x)[NI], double (&y)[NO]) {
+  constexpr int HI = NI / 2, CI = (NI + 1) / 2, HO = NO / 2, CO = (NO + 1) / 2;
+  double a[CO], b[CO];
 #pragma unroll
-  for (int o = 0; o < NO; ++o) y[o] = A[o * NI] * x[0];
+  for (int o = 0; o < CO; ++o) a[o] = b[o] = 0.0;
 #pragma unroll
-  for (int l = 1; l < NI; ++l)
+  for (int l = 0; l < HI; ++l) {
+    const double e = x[l] + x[NI - 1 - l], d = x[l] - x[NI - 1 - l];
 #pragma unroll
-    for (int o = 0; o < NO; ++o) y[o] = fma(A[o * NI + l], x[l], y[o]);
+    for (int o = 0; o < CO; ++o) {
+      a[o] = fma(E[o * CI + l].v, ANTI ? d : e, a[o]);
+      if (o < HO) b[o] = fma(O[o * CI + l].v, ANTI ? e : d, b[o]);
+    }
+  }
+  if (NI & 1) {
+    // the middle entry is even: it joins the even sums (ANTI: the odd ones)
+#pragma unroll
+    for (int o = 0; o < CO; ++o) {
+      if (!ANTI) a[o] = fma(E[o * CI + HI].v, x[HI], a[o]);
+      if (ANTI && o < HO) b[o] = fma(O[o * CI + HI].v, x[HI], b[o]);
+    }
+  }
+#pragma unroll
+  for (int o = 0; o < HO; ++o) {
+    y[o] = a[o] + b[o];
+    y[NO - 1 - o] = a[o] - b[o];
+  }
+  if (NO & 1) y[HO] = a[HO];
 }
 
 template <int L>
@@ -94,10 +149,10 @@ __device__ __forceinline__ void load_line(const double* p, int stride, double (&
   for (int l = 0; l < L; ++l) x[l] = p[l * stride];
 }
 
-// contiguous line (stride 1) at a 16-byte aligned address
-template <int L>
-__device__ __forceinline__ void load_line_v(const double* p, double (&x)[L]) {
-  if constexpr (L % 2 == 0) {
+// contiguous line (stride 1); V: at a 16-byte aligned address, even length
+template <int L, bool V>
+__device__ __forceinline__ void load_row(const double* p, double (&x)[L]) {
+  if constexpr (V) {
 #pragma unroll
     for (int l = 0; l < L; l += 2) {
       const double2 v = *reinterpret_cast<const double2*>(p + l);
@@ -116,173 +171,283 @@ __device__ __forceinline__ void store_line(double* p, int stride, const double (
   for (int l = 0; l < L; ++l) p[l * stride] = x[l];
 }
 
-// n^3 field (global, [k][j][i]) -> m^3 field (shared, rows RM, planes M RM)
-template <int N, int M>
-__device__ __forceinline__ void interpolate_field(const ConvMats<N, M>& mt,
-                                                  const double* __restrict__ src,
-                                                  double* t1, double* t2, double* dst) {
-  using Lay = ConvLayout<N, M>;
-  constexpr int RM = Lay::RM;
-  // x: lines (j, k) of n points -> m points, T1[k][j][o]
-  for (int t = threadIdx.x; t < N * N; t += blockDim.x) {
+template <int L, bool V>
+__device__ __forceinline__ void store_row(double* p, const double (&x)[L]) {
+  if constexpr (V) {
+#pragma unroll
+    for (int l = 0; l < L; l += 2)
+      *reinterpret_cast<double2*>(p + l) = make_double2(x[l], x[l + 1]);
+  } else {
+#pragma unroll
+    for (int l = 0; l < L; ++l) p[l] = x[l];
+  }
+}
+
+// nf fields (field f at src0 for f < 3, src1 for f >= 3, components `cs`
+// apart; n^3 in global) interpolated into dst (fields FM apart), in place
+// stage by stage; ends with a barrier
+template <int N>
+__device__ __forceinline__ void conv_interpolate(const ConvMats<N, ConvLine<N>::M>& mt, int nf,
+                                                 const double* __restrict__ src0,
+                                                 const double* __restrict__ src1, size_t cs,
+                                                 double* dst) {
+  using L = ConvLine<N>;
+  constexpr int M = L::M, RM = L::RM, PL = L::PL, FM = L::FM;
+  // x: lines (j, k) of n points in global memory -> row (k, j) of m points
+  for (int t = threadIdx.x; t < nf * N * N; t += blockDim.x) {
+    const int f = t / (N * N), jk = t - f * (N * N), j = jk % N, k = jk / N;
+    const double* s = (f < 3 ? src0 + f * cs : src1 + (f - 3) * cs) + jk * N;
     double x[N], y[M];
-    if constexpr (N % 2 == 0)
-      load_line_v<N>(src + t * N, x);
-    else
-      load_line<N>(src + t * N, 1, x);
-    line_contract<N, M>(mt.J, x, y);
-    store_line<M>(t1 + t * RM, 1, y);
+    load_row<N, N % 2 == 0>(s, x);
+    eo_contract<N, M, false>(mt.JE, mt.JO, x, y);
+    store_row<M, RM % 2 == 0>(dst + f * FM + k * PL + j * RM, y);
   }
   __syncthreads();
-  // y: lines (o1, k) along j -> T2[k][o2][o1]
-  for (int t = threadIdx.x; t < M * N; t += blockDim.x) {
-    const int o1 = t % M, k = t / M;
+  // y: columns (i, k) along j
+  for (int t = threadIdx.x; t < nf * N * M; t += blockDim.x) {
+    const int f = t / (N * M), r = t - f * (N * M), i = r % M, k = r / M;
+    double* p = dst + f * FM + k * PL + i;
     double x[N], y[M];
-    load_line<N>(t1 + k * N * RM + o1, RM, x);
-    line_contract<N, M>(mt.J, x, y);
-    store_line<M>(t2 + k * M * RM + o1, RM, y);
+    load_line<N>(p, RM, x);
+    eo_contract<N, M, false>(mt.JE, mt.JO, x, y);
+    store_line<M>(p, RM, y);
   }
   __syncthreads();
-  // z: lines (o1, o2) along k -> dst[o3][o2][o1]
-  for (int t = threadIdx.x; t < M * M; t += blockDim.x) {
-    const int o1 = t % M, o2 = t / M;
+  // z: columns (i, j) along k
+  for (int t = threadIdx.x; t < nf * M * M; t += blockDim.x) {
+    const int f = t / (M * M), r = t - f * (M * M), i = r % M, j = r / M;
+    double* p = dst + f * FM + j * RM + i;
     double x[N], y[M];
-    load_line<N>(t2 + o2 * RM + o1, M * RM, x);
-    line_contract<N, M>(mt.J, x, y);
-    store_line<M>(dst + o2 * RM + o1, M * RM, y);
+    load_line<N>(p, PL, x);
+    eo_contract<N, M, false>(mt.JE, mt.JO, x, y);
+    store_line<M>(p, PL, y);
   }
   __syncthreads();
 }
 
-// one direction b of the skew-symmetric form for advected component vc:
-// lines along b; SK (=/+=) A_b d_b vc + B_b d_b(u_b vc) at every point
-template <int N, int M, int B>
-__device__ __forceinline__ void convection_pass(const ConvMats<N, M>& mt,
-                                                const double* __restrict__ W,
-                                                size_t wstride, const double* ui,
-                                                const double* vc, double* sk) {
-  using Lay = ConvLayout<N, M>;
-  constexpr int RM = Lay::RM, FM = Lay::FM;
+// direction B of the skew-symmetric form for nc advected components: SK_c
+// (=, +=) A_b d_b v_c + B_b d_b(u_b v_c) at every point, one line of one
+// component per thread.  AFF: cw = the element's three constants W[.][b]
+// (without the quadrature weights); else Wb = the three per-point arrays.
+template <int N, int B, bool AFF>
+__device__ __forceinline__ void conv_pass(const ConvMats<N, ConvLine<N>::M>& mt, int nc,
+                                          const double* U, const double* V, double* SK,
+                                          double* AB, const double* __restrict__ Wb,
+                                          size_t ws) {
+  using L = ConvLine<N>;
+  constexpr int M = L::M, RM = L::RM, PL = L::PL, FM = L::FM;
   // line step in shared memory / in the unpadded global point index
-  constexpr int SS = B == 0 ? 1 : (B == 1 ? RM : M * RM);
+  constexpr int SS = B == 0 ? 1 : (B == 1 ? RM : PL);
   constexpr int SG = B == 0 ? 1 : (B == 1 ? M : M * M);
-  for (int t = threadIdx.x; t < M * M; t += blockDim.x) {
-    const int a0 = t % M, a1 = t / M;   // the two coordinates across the line
-    int base_s, base_g;
-    if constexpr (B == 0) {            // (j, k)
-      base_s = a0 * RM + a1 * M * RM;
-      base_g = a0 * M + a1 * M * M;
-    } else if constexpr (B == 1) {     // (i, k)
-      base_s = a0 + a1 * M * RM;
-      base_g = a0 + a1 * M * M;
-    } else {                           // (i, j)
-      base_s = a0 + a1 * RM;
-      base_g = a0 + a1 * M;
+  if constexpr (!AFF && L::AB) {
+    // up to six points a thread with every weight load in flight
+    constexpr int MT = M * M * M, RND = (MT + L::THREADS - 1) / L::THREADS, G = RND < 6 ? RND : 6;
+    for (int g0 = threadIdx.x; g0 < MT; g0 += G * L::THREADS) {
+      double w[G][3];
+#pragma unroll
+      for (int h = 0; h < G; ++h) {
+        const int g = g0 + h * L::THREADS;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) w[h][c] = g < MT ? __ldg(Wb + c * ws + g) : 0.0;
+      }
+#pragma unroll
+      for (int h = 0; h < G; ++h) {
+        const int g = g0 + h * L::THREADS;
+        if (g < MT) {
+          const int i = g % M, j = (g / M) % M, k = g / (M * M), q = k * PL + j * RM + i;
+          double A = w[h][0] * U[q];
+          A = fma(w[h][1], U[FM + q], A);
+          AB[q] = fma(w[h][2], U[2 * FM + q], A);
+          AB[FM + q] = (w[h][0] + w[h][1]) + w[h][2];
+        }
+      }
     }
-    double v[M], p[M];
+    __syncthreads();
+  }
+  for (int t = threadIdx.x; t < nc * M * M; t += blockDim.x) {
+    const int c = t / (M * M), r = t - c * (M * M);
+    const int a0 = r % M, a1 = r / M;   // the two coordinates across the line
+    const int bs = B == 0 ? a0 * RM + a1 * PL : (B == 1 ? a0 + a1 * PL : a0 + a1 * RM);
+    const double* vl = V + c * FM + bs;
+    double v[M], ub[M], dv[M], dp[M];
     if constexpr (B == 0) {
-      load_line_v<M>(vc + base_s, v);
-      load_line_v<M>(ui + base_s, p);
+      load_row<M, RM % 2 == 0>(vl, v);
+      load_row<M, RM % 2 == 0>(U + bs, ub);
     } else {
-      load_line<M>(vc + base_s, SS, v);
-      load_line<M>(ui + B * FM + base_s, SS, p);
+      load_line<M>(vl, SS, v);
+      load_line<M>(U + B * FM + bs, SS, ub);
     }
-    double dv[M];
-    line_contract<M, M>(mt.D, v, dv);
+    eo_contract<M, M, true>(mt.DE, mt.DO, v, dv);
 #pragma unroll
-    for (int o = 0; o < M; ++o) p[o] = p[o] * v[o];
-    double dp[M];
-    line_contract<M, M>(mt.D, p, dp);
-#pragma unroll
-    for (int o = 0; o < M; ++o) {
-      const int q = base_s + o * SS;
-      const size_t g = base_g + o * SG;
-      const double w0 = __ldg(W + g), w1 = __ldg(W + wstride + g),
-                   w2 = __ldg(W + 2 * wstride + g);
-      double A = w0 * ui[q];
-      A = fma(w1, ui[FM + q], A);
-      A = fma(w2, ui[2 * FM + q], A);
+    for (int o = 0; o < M; ++o) v[o] = ub[o] * v[o];
+    eo_contract<M, M, true>(mt.DE, mt.DO, v, dp);
+    double* sk = SK + c * FM + bs;
+    if constexpr (AFF) {
+      const double w0 = Wb[0], w1 = Wb[1], w2 = Wb[2];
+      const double wb = B == 0 ? w0 : (B == 1 ? w1 : w2);
       const double Bb = (w0 + w1) + w2;
-      double s = A * dv[o];
-      s = fma(Bb, dp[o], s);
-      if constexpr (B == 0)
-        sk[q] = s;
-      else
-        sk[q] += s;
+      if ((B == 0 || w0 == 0.0) && (B == 1 || w1 == 0.0) && (B == 2 || w2 == 0.0)) {
+        // axis-aligned element: u_b is the only component along b
+#pragma unroll
+        for (int o = 0; o < M; ++o) {
+          const double s = wb * fma(ub[o], dv[o], dp[o]);
+          if (B == 0)
+            sk[o * SS] = s;
+          else
+            sk[o * SS] += s;
+        }
+      } else {
+#pragma unroll
+        for (int o = 0; o < M; ++o) {
+          const double* q = U + bs + o * SS;
+          double A = w0 * q[0];
+          A = fma(w1, q[FM], A);
+          A = fma(w2, q[2 * FM], A);
+          double s = A * dv[o];
+          s = fma(Bb, dp[o], s);
+          if (B == 0)
+            sk[o * SS] = s;
+          else
+            sk[o * SS] += s;
+        }
+      }
+    } else if constexpr (L::AB) {
+      const double* q = AB + bs;
+#pragma unroll
+      for (int o = 0; o < M; ++o) {
+        double s = q[o * SS] * dv[o];
+        s = fma(q[FM + o * SS], dp[o], s);
+        if (B == 0)
+          sk[o * SS] = s;
+        else
+          sk[o * SS] += s;
+      }
+    } else {
+      const int bg = B == 0 ? a0 * M + a1 * M * M : (B == 1 ? a0 + a1 * M * M : a0 + a1 * M);
+#pragma unroll
+      for (int o = 0; o < M; ++o) {
+        const double* q = U + bs + o * SS;
+        const size_t g = bg + o * SG;
+        const double w0 = __ldg(Wb + g), w1 = __ldg(Wb + ws + g), w2 = __ldg(Wb + 2 * ws + g);
+        double A = w0 * q[0];
+        A = fma(w1, q[FM], A);
+        A = fma(w2, q[2 * FM], A);
+        const double Bb = (w0 + w1) + w2;
+        double s = A * dv[o];
+        s = fma(Bb, dp[o], s);
+        if (B == 0)
+          sk[o * SS] = s;
+        else
+          sk[o * SS] += s;
+      }
     }
   }
   __syncthreads();
 }
 
-// m^3 shared field -> n^3 global field through (J^T)^3
-template <int N, int M>
-__device__ __forceinline__ void project_field(const ConvMats<N, M>& mt, const double* sk,
-                                              double* p1, double* p2,
-                                              double* __restrict__ dst) {
-  using Lay = ConvLayout<N, M>;
-  constexpr int RM = Lay::RM, RN = Lay::RN;
-  // i: lines (j, k) of m points -> n points, P1[k][j][p]
-  for (int t = threadIdx.x; t < M * M; t += blockDim.x) {
-    const int j = t % M, k = t / M;
+// nc fields of SK -> out (n^3 in global, components `cs` apart) through
+// (J^T)^3, in place; no barrier at the end (the last stage reads SK only)
+template <int N>
+__device__ __forceinline__ void conv_project(const ConvMats<N, ConvLine<N>::M>& mt, int nc,
+                                             double* SK, double* __restrict__ out, size_t cs) {
+  using L = ConvLine<N>;
+  constexpr int M = L::M, RM = L::RM, PL = L::PL, FM = L::FM;
+  // i: rows (j, k) of m points -> n points
+  for (int t = threadIdx.x; t < nc * M * M; t += blockDim.x) {
+    const int c = t / (M * M), r = t - c * (M * M), j = r % M, k = r / M;
+    double* p = SK + c * FM + k * PL + j * RM;
     double x[M], y[N];
-    load_line_v<M>(sk + j * RM + k * M * RM, x);
-    line_contract<M, N>(mt.JT, x, y);
-    store_line<N>(p1 + (k * M + j) * RN, 1, y);
+    load_row<M, RM % 2 == 0>(p, x);
+    eo_contract<M, N, false>(mt.PE, mt.PO, x, y);
+    store_line<N>(p, 1, y);
   }
   __syncthreads();
-  // j: lines (p1, k) -> P2[k][p2][p1]
-  for (int t = threadIdx.x; t < N * M; t += blockDim.x) {
-    const int q1 = t % N, k = t / N;
+  // j: columns (i, k)
+  for (int t = threadIdx.x; t < nc * N * M; t += blockDim.x) {
+    const int c = t / (N * M), r = t - c * (N * M), i = r % N, k = r / N;
+    double* p = SK + c * FM + k * PL + i;
     double x[M], y[N];
-    load_line<M>(p1 + k * M * RN + q1, RN, x);
-    line_contract<M, N>(mt.JT, x, y);
-    store_line<N>(p2 + k * N * RN + q1, RN, y);
+    load_line<M>(p, RM, x);
+    eo_contract<M, N, false>(mt.PE, mt.PO, x, y);
+    store_line<N>(p, RM, y);
   }
   __syncthreads();
-  // k: lines (p1, p2) -> dst[p3][p2][p1]
-  for (int t = threadIdx.x; t < N * N; t += blockDim.x) {
-    const int q1 = t % N, q2 = t / N;
+  // k: columns (i, j) -> out
+  for (int t = threadIdx.x; t < nc * N * N; t += blockDim.x) {
+    const int c = t / (N * N), r = t - c * (N * N), i = r % N, j = r / N;
     double x[M], y[N];
-    load_line<M>(p2 + q2 * RN + q1, N * RN, x);
-    line_contract<M, N>(mt.JT, x, y);
-    store_line<N>(dst + q2 * N + q1, N * N, y);
+    load_line<M>(SK + c * FM + j * RM + i, PL, x);
+    eo_contract<M, N, false>(mt.PE, mt.PO, x, y);
+    store_line<N>(out + c * cs + r, N * N, y);
   }
-  __syncthreads();
 }
-
-constexpr int kConvThreads = 160;
 
 // Fields u, v, udv hold `nel` elements (component stride nel n^3); the
-// dealiasing factors W hold all `nel_fac` elements of the mesh, and field
-// element e reads the factors of mesh element e0 + e.  W: 9 arrays in the
-// order (b, a), W[(3b + a)][e][q] = rho J tinv[a][b] / 2.
-template <int N, int M>
-__global__ void __launch_bounds__(kConvThreads, 2)
-    k_convection(int nel, int e0, int nel_fac, const double* __restrict__ u,
-                 const double* __restrict__ v, double* __restrict__ udv,
-                 const double* __restrict__ W, const __grid_constant__ ConvMats<N, M> mt) {
-  using Lay = ConvLayout<N, M>;
+// factors hold all elements of the mesh, and field element e uses those of
+// mesh element e0 + e.  W: AFF: 9 constants an element, W[9 e + 3 b + a] =
+// J tinv[a][b] / 2; else 9 arrays of nel_fac m^3, W[(3b + a)][e][q] = rho J
+// tinv[a][b] / 2.  u == v (self-convection): the fields are interpolated
+// once.
+template <int N, bool AFF>
+__global__ void __launch_bounds__(ConvLine<N>::THREADS, ConvLine<N>::BLOCKS)
+    k_conv_line(int nel, int e0, int nel_fac, const double* __restrict__ u,
+                const double* __restrict__ v, double* __restrict__ udv,
+                const double* __restrict__ W, double* __restrict__ scratch,
+                const __grid_constant__ ConvMats<N, ConvLine<N>::M> mt) {
+  using L = ConvLine<N>;
+  constexpr int NT = N * N * N, M = L::M, FM = L::FM, NB = L::NB;
+  constexpr size_t MT = (size_t)M * M * M;
   extern __shared__ __align__(16) double smem[];
-  double* ui = smem;                 // 3 x FM
-  double* vc = ui + 3 * Lay::FM;     // FM; projection stage 1 reuses it
-  double* sk = vc + Lay::FM;         // FM
-  double* t1 = sk + Lay::FM;
-  double* t2 = t1 + Lay::T1;         // projection stage 2 reuses it
-  constexpr int NT = N * N * N, MT = M * M * M;
-  const size_t nptsn = (size_t)nel * NT, wstride = (size_t)nel_fac * MT;
+  double* const U = smem;
+  double* const SK = L::GSK ? scratch + (size_t)blockIdx.x * NB * FM : U + (3 + NB) * FM;
+  double* const AB = U + (3 + (L::GSK ? 1 : 2) * NB) * FM;
+  const bool self = u == v;
+  const size_t cs = (size_t)nel * NT, ws = AFF ? 1 : (size_t)nel_fac * MT;
   for (int e = blockIdx.x; e < nel; e += gridDim.x) {
-    const double* Wb = W + (size_t)(e0 + e) * MT;
-#pragma unroll 1
-    for (int f = 0; f < 3; ++f)
-      interpolate_field<N, M>(mt, u + f * nptsn + (size_t)e * NT, t1, t2, ui + f * Lay::FM);
-#pragma unroll 1
-    for (int c = 0; c < 3; ++c) {
-      interpolate_field<N, M>(mt, v + c * nptsn + (size_t)e * NT, t1, t2, vc);
-      convection_pass<N, M, 0>(mt, Wb, wstride, ui, vc, sk);
-      convection_pass<N, M, 1>(mt, Wb + 3 * wstride, wstride, ui, vc, sk);
-      convection_pass<N, M, 2>(mt, Wb + 6 * wstride, wstride, ui, vc, sk);
-      project_field<N, M>(mt, sk, vc, t2, udv + c * nptsn + (size_t)e * NT);
+    // the next element's fields (and weights) into L2 while this one
+    // computes (a hint: 16-byte aligned chunks only)
+    const int en = e + gridDim.x;
+    if (threadIdx.x < 32 && en < nel) {
+      const int lane = threadIdx.x;
+      const double* p = nullptr;
+      unsigned bytes = NT * sizeof(double);
+      if (lane < 3) {
+        p = u + (size_t)en * NT + lane * cs;
+      } else if (lane < 6) {
+        if (!self) p = v + (size_t)en * NT + (lane - 3) * cs;
+      } else if (!AFF && lane < 15) {
+        p = W + (size_t)(e0 + en) * MT + (lane - 6) * ws;
+        bytes = MT * sizeof(double);
+      }
+      if (p && ((reinterpret_cast<uintptr_t>(p) | bytes) & 15u) == 0) bulk_prefetch_l2(p, bytes);
     }
+    const double* Wb = AFF ? W + 9 * (size_t)(e0 + e) : W + (size_t)(e0 + e) * MT;
+    const double* ue = u + (size_t)e * NT;
+    const double* ve = v + (size_t)e * NT;
+    double* oe = udv + (size_t)e * NT;
+    if constexpr (NB == 3) {
+      double* const V = self ? U : U + 3 * FM;
+      conv_interpolate<N>(mt, self ? 3 : 6, ue, ve, cs, U);
+      conv_pass<N, 0, AFF>(mt, 3, U, V, SK, AB, Wb, ws);
+      conv_pass<N, 1, AFF>(mt, 3, U, V, SK, AB, Wb + 3 * ws, ws);
+      conv_pass<N, 2, AFF>(mt, 3, U, V, SK, AB, Wb + 6 * ws, ws);
+      conv_project<N>(mt, 3, SK, oe, cs);
+    } else {
+      conv_interpolate<N>(mt, 3, ue, ue, cs, U);
+#pragma unroll 1
+      for (int c = 0; c < 3; ++c) {
+        double* const V = self ? U + c * FM : U + 3 * FM;
+        if (!self) conv_interpolate<N>(mt, 1, ve + c * cs, ve, cs, V);
+        conv_pass<N, 0, AFF>(mt, 1, U, V, SK, AB, Wb, ws);
+        conv_pass<N, 1, AFF>(mt, 1, U, V, SK, AB, Wb + 3 * ws, ws);
+        conv_pass<N, 2, AFF>(mt, 1, U, V, SK, AB, Wb + 6 * ws, ws);
+        conv_project<N>(mt, 1, SK, oe + c * cs, cs);
+        // the next component's first pass writes SK, its interpolation V
+        if (self) __syncthreads();
+      }
+    }
+    // the next element's interpolation writes U and V, last read before the
+    // projection's barriers; its first pass writes SK after three barriers
   }
 }
 
@@ -393,82 +558,100 @@ static size_t convection_rt_smem(int n, int m, bool fields) {
 
 static constexpr size_t kConvSmemMax = 227 * 1024;
 
-template <int N>
-static constexpr bool conv_fast_order() {
-  return dev::conv_smem_bytes<N, (3 * N) / 2>() <= kConvSmemMax;
-}
-
-static bool conv_fast(int n, int m) {
-  if (m != (3 * n) / 2) return false;
-  switch (n) {
-#define SSG_CONVF(NV) \
-  case NV:            \
-    return conv_fast_order<NV>();
-    SSG_CONVF(2) SSG_CONVF(3) SSG_CONVF(4) SSG_CONVF(5) SSG_CONVF(6) SSG_CONVF(7)
-    SSG_CONVF(8) SSG_CONVF(9) SSG_CONVF(10) SSG_CONVF(11)
-#undef SSG_CONVF
-    default:
-      return false;
-  }
-}
-
 size_t convection_scratch_doubles(int n, int m) {
-  if (conv_fast(n, m) || convection_rt_smem(n, m, true) <= kConvSmemMax) return 0;
+  if (convection_rt_smem(n, m, true) <= kConvSmemMax) return 0;
   return (size_t)kConvScratchBlocks * 5 * m * m * m;
 }
 
+// even / odd halves of A (no x ni, A[o * ni + i]); false when A is not
+// (anti)symmetric under reversal of both indices to rounding
+bool conv_eo_split(int ni, int no, const double* A, bool anti, std::vector<double>& E,
+                   std::vector<double>& O) {
+  const int ci = (ni + 1) / 2, co = (no + 1) / 2;
+  E.assign((size_t)co * ci, 0.0);
+  O.assign((size_t)co * ci, 0.0);
+  const double sg = anti ? -1.0 : 1.0;
+  double top = 0.0;
+  for (int q = 0; q < ni * no; ++q) top = std::max(top, std::fabs(A[q]));
+  std::vector<double> S((size_t)ni * no);
+  for (int o = 0; o < no; ++o)
+    for (int i = 0; i < ni; ++i) {
+      const double a = A[o * ni + i], b = sg * A[(no - 1 - o) * ni + ni - 1 - i];
+      if (!(std::fabs(a - b) <= 1e-13 * top)) return false;
+      S[o * ni + i] = 0.5 * (a + b);
+    }
+  for (int o = 0; o < co; ++o)
+    for (int i = 0; i < ci; ++i) {
+      const double p = S[o * ni + i], q = S[o * ni + ni - 1 - i];
+      const bool mid = 2 * i + 1 == ni;
+      // even inputs weigh (p + q) / 2, odd ones (p - q) / 2; E multiplies the
+      // part that the reversal keeps (even, or odd when antisymmetric)
+      const double even = mid ? p : 0.5 * (p + q), odd = 0.5 * (p - q);
+      E[o * ci + i] = anti ? odd : even;
+      O[o * ci + i] = anti ? even : odd;
+    }
+  return true;
+}
+
 template <int N>
-static cudaError_t launch_fast(cudaStream_t s, int nel, int e0, int nel_fac, const double* u,
-                               const double* v, double* udv, const double* W,
-                               const double* Dh, const double* Jh, int grid) {
-  constexpr int M = (3 * N) / 2;
-  if constexpr (!conv_fast_order<N>()) {
-    return cudaErrorInvalidValue;
-  } else {
-    dev::ConvMats<N, M> mt;
-    for (int q = 0; q < M * M; ++q) mt.D[q] = Dh[q];
-    for (int o = 0; o < M; ++o)
-      for (int p = 0; p < N; ++p) {
-        mt.J[o * N + p] = Jh[o * N + p];
-        mt.JT[p * M + o] = Jh[o * N + p];
-      }
-    constexpr size_t smem = dev::conv_smem_bytes<N, M>();
+static cudaError_t launch_line(cudaStream_t s, int nel, int e0, int nel_fac, const double* u,
+                               const double* v, double* udv, const ConvGeom& g) {
+  using L = dev::ConvLine<N>;
+  constexpr int M = L::M;
+  dev::ConvMats<N, M> mt = {};
+  auto put = [](dev::ConvEntry* dst, const double* src, size_t count) {
+    for (size_t q = 0; q < count; ++q) dst[q].v = src[q];
+  };
+  put(mt.JE, g.eo[0], std::size(mt.JE));
+  put(mt.JO, g.eo[1], std::size(mt.JO));
+  put(mt.DE, g.eo[2], std::size(mt.DE));
+  put(mt.DO, g.eo[3], std::size(mt.DO));
+  put(mt.PE, g.eo[4], std::size(mt.PE));
+  put(mt.PO, g.eo[5], std::size(mt.PO));
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  auto go = [&](auto aff) -> cudaError_t {
+    constexpr bool A = decltype(aff)::value;
+    auto kern = &dev::k_conv_line<N, A>;
     static SmemAttr attr;
-    cudaError_t e = attr.ensure((const void*)dev::k_convection<N, M>, smem);
-    if (e != cudaSuccess) return e;
+    cudaError_t ce = attr.ensure((const void*)kern, L::smem(A));
+    if (ce != cudaSuccess) return ce;
+    // one wave of resident blocks walking the elements
+    constexpr int fit = (int)(kConvSmemMax / L::smem(A));
+    constexpr int per = fit < 1 ? 1 : (fit > 8 ? 8 : fit);
+    const int grid = std::min(std::min(nel, per * sms), L::GSK ? kConvScratchBlocks : nel);
     count_launch();
-    dev::k_convection<N, M><<<grid, dev::kConvThreads, smem, s>>>(nel, e0, nel_fac, u, v, udv,
-                                                                 W, mt);
+    kern<<<grid, L::THREADS, L::smem(A), s>>>(nel, e0, nel_fac, u, v, udv, A ? g.aff : g.W,
+                                            g.scratch, mt);
     return cudaGetLastError();
-  }
+  };
+  return g.aff ? go(std::true_type()) : go(std::false_type());
 }
 
 cudaError_t run_convection(cudaStream_t s, int nel, int e0, int nel_fac, int n, int m,
-                           const double* u, const double* v, double* udv, const double* W,
-                           const double* Dh, const double* Jh, const double* Dd,
-                           const double* Jd, double* scratch) {
+                           const double* u, const double* v, double* udv, const ConvGeom& g) {
   if (nel <= 0) return cudaSuccess;
-  if (convection_dmma_applies(n, m))
-    return run_convection_dmma(s, nel, e0, nel_fac, u, v, udv, W, Dh, Jh);
-  // the compile-time-order kernel reads element lines with 16-byte loads:
-  // fields at addresses that are not 16-byte aligned take the runtime-order
-  // kernel
+  // even orders read element lines with 16-byte loads: fields at addresses
+  // that are not 16-byte aligned take the runtime-order kernel
   const bool aligned =
       ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(v)) & 15u) == 0;
-  if (aligned && conv_fast(n, m)) {
+  if (aligned && g.eo[0] && m == (3 * n) / 2 && (n < 12 || g.scratch)) {
     switch (n) {
 #define SSG_CONVL(NV) \
   case NV:            \
-    return launch_fast<NV>(s, nel, e0, nel_fac, u, v, udv, W, Dh, Jh, nel);
+    return launch_line<NV>(s, nel, e0, nel_fac, u, v, udv, g);
       SSG_CONVL(2) SSG_CONVL(3) SSG_CONVL(4) SSG_CONVL(5) SSG_CONVL(6) SSG_CONVL(7)
-      SSG_CONVL(8) SSG_CONVL(9) SSG_CONVL(10) SSG_CONVL(11)
+      SSG_CONVL(8) SSG_CONVL(9) SSG_CONVL(10) SSG_CONVL(11) SSG_CONVL(12)
 #undef SSG_CONVL
       default:
         break;
     }
   }
   const bool in_smem = convection_rt_smem(n, m, true) <= kConvSmemMax;
-  if (!in_smem && !scratch) return cudaErrorInvalidValue;
+  if (!in_smem && !g.scratch) return cudaErrorInvalidValue;
   const size_t smem = convection_rt_smem(n, m, in_smem);
   if (smem > kConvSmemMax) return cudaErrorInvalidValue;
   static SmemAttr attr;
@@ -478,8 +661,8 @@ cudaError_t run_convection(cudaStream_t s, int nel, int e0, int nel_fac, int n, 
   }
   const int grid = in_smem ? nel : std::min(nel, kConvScratchBlocks);
   count_launch();
-  dev::k_convection_rt<<<grid, 512, smem, s>>>(nel, e0, nel_fac, n, m, u, v, udv, W, Dd, Jd,
-                                               in_smem ? nullptr : scratch);
+  dev::k_convection_rt<<<grid, 512, smem, s>>>(nel, e0, nel_fac, n, m, u, v, udv, g.W, g.Dd,
+                                               g.Jd, in_smem ? nullptr : g.scratch);
   return cudaGetLastError();
 }
 

@@ -349,8 +349,7 @@ ssg_status ssg_navier_stokes_step(ssg_context* c, const double* f, const double*
   // lagrangian_convection_integration
   rotate(c->fconv);
   SSG_CUDA(c, run_convection(s, c->nel, 0, c->nel, c->n, c->m, c->fu[0], c->fu[0], c->fconv[0],
-                             c->conv_w, c->host.conv.D.data(), c->host.jconv.data(), c->conv_D,
-                             c->conv_J, c->conv_scratch));
+                             conv_geom(c)));
   SSG_CUDA(c, cudaMemsetAsync(c->fut, 0, 3 * np * sizeof(double), s));
   const double tt[4] = {t - 2.0 * dt, t - dt, t, t + dt};
   const double beta[3] = {1.0 / 3.0, -3.0 / 2.0, 3.0};

@@ -480,18 +480,25 @@ static void element_constants(int n, int nel, size_t nt, int nf, const double* c
   parallel_elements(nel, [&](int e0, int e1) {
     for (int e = e0; e < e1 && affine.load(std::memory_order_relaxed); ++e) {
       const size_t o = (size_t)e * nt;
-      double mean[9], top = 0.0;
+      double mean[9], lo[9], hi[9], top = 0.0;
       for (int a = 0; a < nf; ++a) {
-        double s = 0.0;
-        for (size_t q = 0; q < nt; ++q) s += f[a][o + q] * det[o + q];
+        double s = 0.0, mn = f[a][o] * det[o], mx = mn;
+        for (size_t q = 0; q < nt; ++q) {
+          const double v = f[a][o + q] * det[o + q];
+          s += v;
+          mn = v < mn ? v : mn;
+          mx = v > mx ? v : mx;
+        }
         mean[a] = s / (double)nt;
+        lo[a] = mn;
+        hi[a] = mx;
         top = std::max(top, std::fabs(mean[a]));
       }
+      // (a NaN among the factors makes its mean, and top or the test, NaN)
       const double tol = noise * top;
       bool ok = std::isfinite(top) && top > 0.0;
-      for (int a = 0; a < nf && ok; ++a)
-        for (size_t q = 0; q < nt; ++q)
-          if (!(std::fabs(f[a][o + q] * det[o + q] - mean[a]) <= tol)) ok = false;
+      for (int a = 0; a < nf; ++a)
+        ok = ok && hi[a] - mean[a] <= tol && mean[a] - lo[a] <= tol;
       if (!ok) affine.store(false, std::memory_order_relaxed);
       for (int a = 0; a < nf; ++a)
         c[(size_t)nf * e + a] = std::fabs(mean[a]) <= tol ? 0.0 : mean[a];
@@ -504,6 +511,14 @@ void affine_metric(const HostLevel& L, int nel, std::vector<double>& c) {
   const double* g[6];
   for (int a = 0; a < 6; ++a) g[a] = L.g[a].data();
   element_constants(L.n, nel, L.nt, 6, g, L.det.data(), c);
+}
+
+void affine_convection(const HostLevel& L, int nel, std::vector<double>& c) {
+  const double* t[9];
+  for (int b = 0; b < 3; ++b)
+    for (int a = 0; a < 3; ++a) t[3 * b + a] = L.tinv[3 * a + b].data();
+  element_constants(L.n, nel, L.nt, 9, t, L.det.data(), c);
+  for (auto& v : c) v *= 0.5;
 }
 
 // Element-local Jacobi diagonal of the Laplacian in the reference's form

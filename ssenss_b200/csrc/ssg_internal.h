@@ -90,6 +90,8 @@ ssg_status build_pairs(HostMesh& m, std::string& err, bool opposite = false);
 // The constant metric of each element (nel x 6: G_ab J) where every element
 // of the level is an affine image of the reference cube; empty otherwise.
 void affine_metric(const HostLevel& L, int nel, std::vector<double>& c);
+// The same for the convection weights: nel x 9, [3b + a] = J tinv[a][b] / 2.
+void affine_convection(const HostLevel& L, int nel, std::vector<double>& c);
 void stiffness_diagonal(const HostLevel& L, int nel, double* out);
 void host_dss(const HostMesh& m, int n, double* u);
 // DSS map of one level (one int array):
@@ -198,6 +200,8 @@ struct ssg_context {
   double* conv_w = nullptr;     // 9 x nel x m^3: W[3b + a] = rho J tinv[a][b] / 2
   double* conv_D = nullptr;     // m*m
   double* conv_J = nullptr;     // m*n, jconv[i*n+p]
+  double* conv_aff = nullptr;   // 9 x nel constants where every element is affine, else null
+  std::vector<double> conv_eo[6];  // even / odd halves of the matrices (empty: no symmetry)
   double* conv_scratch = nullptr;  // interpolated fields when m^3 exceeds shared memory
   // particles
   double* p_jac = nullptr;      // 9 x npts (level 0)
@@ -267,6 +271,19 @@ ssg_status cuda_fail(ssg_context* c, cudaError_t e, const char* what);
   } while (0)
 
 bool is_device_ptr(const void* p);
+
+// the context's dealiasing data for run_convection
+inline ConvGeom conv_geom(const ssg_context* c) {
+  ConvGeom g;
+  g.W = c->conv_w;
+  g.aff = c->conv_aff;
+  if (!c->conv_eo[0].empty())
+    for (int k = 0; k < 6; ++k) g.eo[k] = c->conv_eo[k].data();
+  g.Dd = c->conv_D;
+  g.Jd = c->conv_J;
+  g.scratch = c->conv_scratch;
+  return g;
+}
 
 enum Frame { FR_LEVEL0 = 0, FR_HELM = 8, FR_FCG = 9, FR_MISC = 10, FR_COUNT = 12 };
 

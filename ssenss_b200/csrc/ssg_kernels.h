@@ -5,6 +5,7 @@
 #include <atomic>
 #include <cstddef>
 #include <cstdint>
+#include <vector>
 
 namespace ssg {
 
@@ -236,21 +237,28 @@ cudaError_t run_coarse_cg(cudaStream_t s, int device, int nel, const double* f, 
 // doubles (0: none needed)
 constexpr int kConvScratchBlocks = 296;
 size_t convection_scratch_doubles(int n, int m);
-// W: 9 x nel_fac x m^3 in the order (b, a), W[3b + a] = rho J tinv[a][b] / 2;
-// Dh, Jh: host copies of the m-point derivative matrix D[i*m + l] and the
-// interpolation matrix J[i*n + p] (carried in the kernel's parameters);
-// Dd, Jd: the same on the device (runtime-order kernel)
+struct ConvGeom {
+  // 9 x nel_fac x m^3 in the order (b, a), W[3b + a] = rho J tinv[a][b] / 2
+  const double* W = nullptr;
+  // every element affine on the dealiasing grid: 9 constants an element,
+  // J tinv[a][b] / 2 in the same order; else null
+  const double* aff = nullptr;
+  // host: even / odd halves of the interpolation matrix, the derivative and
+  // the projection (J^T, with the quadrature weights when affine), each E
+  // then O (conv_eo_split); null where one lacks the symmetry
+  const double* eo[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  // the m-point derivative matrix D[i*m + l] and the interpolation matrix
+  // J[i*n + p] on the device (runtime-order kernel)
+  const double *Dd = nullptr, *Jd = nullptr;
+  double* scratch = nullptr;
+};
+// Even / odd halves of A (no x ni, A[o * ni + i]) for a matrix symmetric
+// (anti: antisymmetric) under reversal of both indices; false when it is
+// not, to rounding
+bool conv_eo_split(int ni, int no, const double* A, bool anti, std::vector<double>& E,
+                   std::vector<double>& O);
 cudaError_t run_convection(cudaStream_t s, int nel, int e0, int nel_fac, int n, int m,
-                           const double* u, const double* v, double* udv, const double* W,
-                           const double* Dh, const double* Jh, const double* Dd,
-                           const double* Jd, double* scratch);
-// Convection at n = 8, m = 12 on the FP64 tensor cores (conv_dmma.cu): the
-// self-convection kernel when u == v, else the general one; run_convection
-// takes them at that order
-bool convection_dmma_applies(int n, int m);
-cudaError_t run_convection_dmma(cudaStream_t s, int nel, int e0, int nel_fac, const double* u,
-                                const double* v, double* udv, const double* W,
-                                const double* Dh, const double* Jh);
+                           const double* u, const double* v, double* udv, const ConvGeom& g);
 // Stokes operators of the time step, one element per block (stokes.cu):
 // which 0 = the double curl of in (3 fields) into out (3 fields); 1 = the
 // pressure right-hand side of in = u~ (3 fields) and g (3 fields, surface

@@ -161,9 +161,7 @@ ssg_status convection_rk4(ssg_context* c, double* du, double t0, double t, doubl
                                              i > 0, ut, uoo, uo, uc, w.a, w.b, w.c, w.fa, w.fb,
                                              w.fc);
       SSG_CUDA(c, cudaGetLastError());
-      SSG_CUDA(c, run_convection(s, c->nel, 0, c->nel, c->n, c->m, ut, y, f[i], c->conv_w,
-                                 c->host.conv.D.data(), c->host.jconv.data(), c->conv_D,
-                                 c->conv_J, c->conv_scratch));
+      SSG_CUDA(c, run_convection(s, c->nel, 0, c->nel, c->n, c->m, ut, y, f[i], conv_geom(c)));
       // trivec_inverse_mass_matrix: per component the DSS, then the product
       // with 1 / DSS(mass), the three components in one pass
       SSG_CUDA(c, run_dss3(s, true, L.n, c->nel, f[i], y, npc, c->d_nbreg, L.dss_ec, c->inv_mass));

@@ -1,4 +1,4 @@
-"""The operator on affine elements (parallelepipeds), where the library holds
+"""The operator and convection on affine elements (parallelepipeds), where the library holds
 six metric constants an element instead of six factors a point, against the
 oracle's per-point factors; and the rule's other side, a mesh with a single
 deformed element, which keeps the per-point factors.
@@ -73,5 +73,85 @@ def test_poisson_on_affine_elements(mesh, n, precision, gpu_ctx_factory):
     res = f - orc.global_opeval(O.PRESSURE, u)
     res -= (w * res).sum() / w.sum()
     assert np.sqrt((w * res * res).sum()) < 1.5e-10 + 4e-14 * n * n * np.sqrt((w * f * f).sum())
+    ctx.close()
+    orc.close()
+
+
+def conv_reference(u, v, J, D, w, det, tinv):
+    """The operator's definition in numpy for given matrices: D on the m
+    points, J (m, n), weights w, det and tinv[a][b] = dr_b/dx_a there."""
+    rho = w[:, None, None] * w[:, None] * w
+    ax = ("pi,ekji->ekjp", "pj,ekji->ekpi", "pk,ekji->epji")
+
+    def to(A, x):
+        for e in ax:
+            x = np.einsum(e, A, x)
+        return x
+
+    ui = [to(J, u[a]) for a in range(3)]
+    out = []
+    for c in range(3):
+        vi = to(J, v[c])
+        s = 0.0
+        for b in range(3):
+            dv, dp = np.einsum(ax[b], D, vi), np.einsum(ax[b], D, ui[b] * vi)
+            for a in range(3):
+                s = s + tinv[3 * a + b] * (ui[a] * dv + dp)
+        out.append(to(J.T, 0.5 * rho * det * s))
+    return np.stack(out)
+
+
+@pytest.mark.parametrize("n", range(2, 13))
+@pytest.mark.parametrize("mesh", ["box", "sheared", "channel"])
+def test_convection_at_every_order(mesh, n, gpu_ctx_factory):
+    """Both forms (u advecting v, and itself) against the oracle: nine
+    constants an element on the affine meshes (to the noise of the oracle's
+    own factors), per-point weights on the channel (1e-13); then the same
+    fields at addresses that are not 16-byte aligned, which take the
+    runtime-order kernel (1e-13 of each other, plus that noise)."""
+    import torch
+    m = {"box": lambda: box_mesh((3, 3, 4)), "sheared": sheared,
+         "channel": lambda: channel_mesh((4, 3, 3), seed=7)}[mesh]()
+    orc = O.Oracle(m, n)
+    ctx = gpu_ctx_factory(m, n)
+    md = (3 * n) // 2
+    tol = 1e-13 if mesh == "channel" else 1e-13 + 4e-14 * md * md
+    rng = np.random.default_rng(n)
+    u = rng.standard_normal((3, m.nel, n, n, n))
+    v = rng.standard_normal((3, m.nel, n, n, n))
+    got = ctx.convection_operator(u, v)
+    assert rel(got, orc.convection(u, v)) < tol
+    assert rel(ctx.convection_operator(u, u), orc.convection(u, u)) < tol
+    raw = torch.zeros(2 * u.size + 2, dtype=torch.float64, device="cuda")
+    um, vm = raw[1:1 + u.size].view(u.shape), raw[1 + u.size:1 + 2 * u.size].view(u.shape)
+    um.copy_(torch.from_numpy(u))
+    vm.copy_(torch.from_numpy(v))
+    torch.cuda.synchronize()
+    out = ctx.convection_operator(um, vm, torch.empty_like(um))
+    assert rel(out.cpu().numpy(), got) < tol
+    ctx.close()
+    orc.close()
+
+
+@pytest.mark.parametrize("n", [5, 8])
+def test_convection_with_matrices_that_are_not_symmetric(n, gpu_ctx_factory):
+    """A caller's own interpolation matrix without the points' symmetry: the
+    line kernel's even / odd split does not apply, the result is the
+    definition's all the same."""
+    m = box_mesh((3, 3, 3))
+    orc = O.Oracle(m, n)
+    ctx = gpu_ctx_factory(m, n)
+    md = (3 * n) // 2
+    rng = np.random.default_rng(5)
+    J = rng.standard_normal((md, n))
+    D = rng.standard_normal((md, md))
+    w = rng.uniform(0.1, 1.0, md)
+    det = rng.uniform(0.5, 1.5, (m.nel, md, md, md))
+    tinv = rng.standard_normal((9, m.nel, md, md, md))
+    # stored matrices: deriv d[j][i] = D_ij, interp n x m
+    ctx.setup_dealias(md, np.ascontiguousarray(D.T), w, tinv, det, np.ascontiguousarray(J.T))
+    u = rng.standard_normal((3, m.nel, n, n, n))
+    v = rng.standard_normal((3, m.nel, n, n, n))
+    assert rel(ctx.convection_operator(u, v), conv_reference(u, v, J, D, w, det, tinv)) < 1e-13
     ctx.close()
     orc.close()
