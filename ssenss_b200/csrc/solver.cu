@@ -269,6 +269,16 @@ static ssg_status read_flag(ssg_context* c, const double* dptr, double* v) {
   return SSG_OK;
 }
 
+// status of a finished CG solve from its frame
+static ssg_status cg_outcome(ssg_context* c, const double* fr, double eps, int max_iter) {
+  double err, iters;
+  SSG_TRY(read_flag(c, fr + F_ERR, &err));
+  SSG_TRY(read_flag(c, fr + F_ITER, &iters));
+  if (!std::isfinite(err)) return fail(c, SSG_NONFINITE, "non-finite CG residual");
+  if (!(err <= eps) && iters >= max_iter) return SSG_MAXITER;
+  return SSG_OK;
+}
+
 ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void* x,
                     double eps, int max_iter, int frame, double* hist, int hist_cap,
                     bool sync_each) {
@@ -298,6 +308,37 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
   op.max_iter = max_iter;
   op.hist = hist;
   op.hist_cap = hist_cap;
+
+  // a level that fits one thread-block cluster: the whole solve in one launch
+  {
+    ClusterCgRun R;
+    R.nel = c->nel;
+    R.helm = helm;
+    R.f = f;
+    R.x = x;
+    R.ex = W.aploc;
+    R.gf = L.n == 8 && !fp32 ? nullptr : gf;
+    R.bj = L.bj;
+    R.D = L.D;
+    R.S = helm ? L.S : L.D;
+    R.lambda = lam;
+    R.dinv = dinv;
+    R.mult = L.mult;
+    R.mask = mask;
+    R.dss = L.dss_ec;
+    R.ag = aff_geom(L);
+    R.nunique = L.nunique;
+    R.eps = eps;
+    R.max_iter = max_iter;
+    R.frame = fr;
+    R.hist = hist;
+    R.hist_cap = hist_cap;
+    bool fits = false;
+    // (n = 8 keeps its FP64 factors in fragment order: affine levels only)
+    if (max_iter > 0 && (R.gf || R.ag.c))
+      SSG_CUDA(c, run_cluster_cg(s, c->device, L.n, fp32, R, true, &fits));
+    if (fits) return sync_each ? cg_outcome(c, fr, eps, max_iter) : SSG_OK;
+  }
 
   // mask f; r = f - A x; subtract_nullspace(r)
   if (mask) SSG_CUDA(c, run_mul(s, fp32, np, f, mask));
@@ -454,12 +495,7 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
     }
   }
   if (!sync_each) return SSG_OK;   // smoother: outcome stays on the device
-  double err, iters;
-  SSG_TRY(read_flag(c, fr + F_ERR, &err));
-  SSG_TRY(read_flag(c, fr + F_ITER, &iters));
-  if (!std::isfinite(err)) return fail(c, SSG_NONFINITE, "non-finite CG residual");
-  if (!(err <= eps) && iters >= max_iter) return SSG_MAXITER;
-  return SSG_OK;
+  return cg_outcome(c, fr, eps, max_iter);
 }
 
 // coarsest level (n = 2): CG-Jacobi, 500 iterations, in one cooperative launch
@@ -471,6 +507,11 @@ static ssg_status coarse_solve(ssg_context* c, int L, double* f, double* x, doub
     return cg_solve(c, L, SSG_PRESSURE, false, f, x, eps, max_iter, FR_LEVEL0 + L, nullptr,
                     0, false);
   }
+  bool done = false;
+  SSG_CUDA(c, run_cluster_coarse(c->stream, c->device, c->nel, f, x, (double*)W.aploc, C.gf,
+                                 C.D, C.dinv_p, c->d_pairs, C.nunique, eps, rel, max_iter,
+                                 c->d_sc + (FR_LEVEL0 + L) * F_SIZE, &done));
+  if (done) return SSG_OK;
   SSG_CUDA(c, run_coarse_cg(c->stream, c->device, c->nel, f, x, (double*)W.r, (double*)W.z,
                             (double*)W.p, (double*)W.aploc, (double*)W.ap, C.gf, C.D,
                             C.dinv_p, C.mult, c->d_pairs, C.nunique, eps, rel, max_iter,
@@ -530,6 +571,14 @@ static ssg_status mg_recurse(ssg_context* c, int L, void* f, void* x, double eps
   // took the outer FCG 16 iterations instead of 11 on the C2 solve.
 
   if (F.n == 4 && !fp32) {
+    // (a level that fits a cluster runs there)
+    ClusterCgRun K;
+    K.nel = c->nel;
+    K.ag = aff_geom(F);
+    bool fits = false;
+    SSG_CUDA(c, run_cluster_cg(s, c->device, F.n, fp32, K, false, &fits));
+    if (fits)
+      return cg_solve(c, L, SSG_PRESSURE, fp32, f, x, eps, 15, FR_LEVEL0 + L, nullptr, 0, false);
     LevelCgRun R;
     R.nel = c->nel;
     R.f = f;

@@ -221,6 +221,36 @@ struct LevelCgRun {
   double* part = nullptr;
   size_t part_cap = 0;
 };
+// Jacobi CG of a small level in one thread-block cluster (cluster.cu): the
+// arithmetic of cg_solve at that level and precision.  launch false: only
+// tells whether the level fits.  fits false: nothing was launched.
+struct ClusterCgRun {
+  int nel = 0;
+  int helm = 0;
+  void *f = nullptr, *x = nullptr;
+  void* ex = nullptr;         // scratch vector (the exchanged operator output)
+  const void* gf = nullptr;
+  const double *bj = nullptr, *D = nullptr, *S = nullptr;
+  double lambda = 0.0;
+  const void* dinv = nullptr;
+  const uint8_t* mult = nullptr;
+  const double* mask = nullptr;
+  const int* dss = nullptr;   // DSS map (dss_map_table)
+  AffGeom ag;
+  double nunique = 1.0, eps = 0.0;
+  int max_iter = 0;
+  double* frame = nullptr;
+  double* hist = nullptr;
+  int hist_cap = 0;
+};
+cudaError_t run_cluster_cg(cudaStream_t s, int device, int n, bool fp32, const ClusterCgRun& L,
+                           bool launch, bool* fits);
+// the n = 2 level in one cluster; done false: it does not fit, nothing was
+// launched
+cudaError_t run_cluster_coarse(cudaStream_t s, int device, int nel, const double* f, double* x,
+                               double* ex, const double* gf, const double* D, const double* dinv,
+                               const int* pairs, double nunique, double eps, double rel,
+                               int max_iter, double* frame, bool* done);
 cudaError_t run_level_cg(cudaStream_t s, int device, int n, bool fp32, const LevelCgRun& L);
 // whole CG-Jacobi solve of an n = 2 level in one cooperative launch
 // (coarse.cu); it stops at sqrt((r.r)_w) <= eps, or <= rel times the first
