@@ -321,6 +321,14 @@ static ssg_status upload_all(ssg_context* c) {
       dss_map_table(H, h.n, ec);
       SSG_TRY(dupload(c, &d.dss_ec, ec.data(), ec.size()));
     }
+    d.sym = true;
+    for (const std::vector<double>* A : {&h.D, &h.S}) {
+      const int n = h.n;
+      double top = 0.0;
+      for (double v : *A) top = std::max(top, std::fabs(v));
+      for (int q = 0; q < n * n; ++q)
+        if (!(std::fabs((*A)[q] + (*A)[n * n - 1 - q]) <= 1e-12 * top)) d.sym = false;
+    }
     SSG_TRY(dupload(c, &d.D, h.D.data(), h.D.size()));
     SSG_TRY(dupload(c, &d.S, h.S.data(), h.S.size()));
     SSG_TRY(upload_f32(c, &d.dinv_p32, dp.data(), np));

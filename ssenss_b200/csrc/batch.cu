@@ -395,7 +395,7 @@ ssg_status seg_solve(ssg_context* c, const SegLevel& L, SegScratch& W, int nseg,
   if (L.mask) SSG_CUDA(c, run_mul(s, false, np, W.f, L.mask));
   auto op = [&](const double* in) -> ssg_status {
     SSG_CUDA(c, run_ax(s, L.n, L.nel, 0, true, false, in, W.aploc, L.gf, np, W.bj_s, L.D, L.S,
-                       1.0, nullptr));
+                       1.0, nullptr, L.ag));
     SSG_CUDA(c, run_dss(s, DSS_PLAIN, false, L.n, L.nel, W.aploc, W.ap, nullptr, L.dss, L.mask,
                         nullptr, nullptr, nullptr));
     return SSG_OK;
@@ -516,6 +516,7 @@ extern "C" ssg_status ssg_solve_helmholtz_segments(ssg_context* c, int var, int 
   L.S = D.S;
   L.mult = D.mult;
   L.dss = D.dss_ec;
+  L.ag = aff_geom(D);
   if (!c->seg) c->seg = new SegScratch();
   return seg_solve(c, L, *c->seg, nseg, seg_first, lambda, f, u, eps, max_iter, info);
 }

@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(256, (N >= 10 ? 1 : 2)) k_ax(int nel, T* __res
 // interface as k_ax (optional direction update and p . (A p)).
 // ---------------------------------------------------------------------------
 template <int N, typename T, bool HELM, bool FUSEP, bool AFF>
-__global__ void __launch_bounds__(AxLine<N>::THREADS)
+__global__ void __launch_bounds__(AxLine<N>::THREADS, axl_blocks<N, T, HELM>())
     k_axl(int nel, T* __restrict__ u, T* __restrict__ au, const T* __restrict__ gf,
           size_t npts, const double* __restrict__ bj, const double* __restrict__ Dg,
           const double* __restrict__ Sg, double lambda, PUpdate pu, ScalarOp dop, AffGeom ag) {
@@ -932,9 +932,10 @@ int vec_blocks(size_t npts) {
   return (int)(b < cap ? (b ? b : 1) : cap);
 }
 
-int ax_epb(int n) {
+int ax_epb(int n, bool sym) {
+  if (sym) return kAxLine;
   if (n >= 0 && n <= SSG_MAXN && g_tune_ax_epb[n].load() != 0) return g_tune_ax_epb[n].load();
-  return kAxLine;
+  return ax_epb_max(n);
 }
 
 // the plane-form (epb > 0 elements per block) or line-form (kAxLine) kernel
@@ -1014,7 +1015,7 @@ cudaError_t run_ax(cudaStream_t s, int n, int nel, int epb, bool helm, bool fp32
   if (dmma)
     return run_ax8_dmma(s, nel, helm, fp32, (void*)in, out, gf, npts, bj, D, S, lambda,
                         fuse ? &pu : nullptr, &dop, ag);
-  if (epb == 0) epb = ax_epb(n);
+  if (epb == 0) epb = ax_epb(n, ag.sym);
   if (fp32) {
     if (helm) return cudaErrorInvalidValue;
     if (fuse)

@@ -542,85 +542,135 @@ __device__ __forceinline__ double ax_element(int e, bool active, int i, int j, c
   return pap;
 }
 
+// A matrix antisymmetric under reversal of both indices (every derivative
+// matrix on the GLL points: A[N-1-o][N-1-l] = -A[o][l]) as its even and odd
+// halves: with e_l = x_l + x_{N-1-l}, d_l = x_l - x_{N-1-l} the outputs are
+// y_o = a_o + b_o, y_{N-1-o} = a_o - b_o, a = E d, b = O e: half the
+// multiply-adds and half the matrix reads.  E[l][o], then O[l][o] (the middle
+// input of an odd order as l = N / 2), outputs pair-aligned.
+template <int N>
+struct EoMat {
+  static constexpr int H = N / 2, C = (N + 1) / 2;
+  static constexpr int EP = C + (C & 1), OP = H + (H & 1);   // row lengths
+  static constexpr int O0 = H * EP, SIZE = O0 + C * OP;
+};
+
 // ---------------------------------------------------------------------------
-// line-form element operator (k_axl in kernels.cu, the fused cooperative
-// smoother in coarse.cu): each thread contracts one whole line of an
-// element (N points along i, j or k) held in registers, so a matrix row is
-// read once per line instead of a shared row and a shared field value per
-// multiply-add.  Per element: the field is staged in shared memory; lines
+// line-form element operator (k_axl in kernels.cu): each thread contracts one
+// whole line of an element (N points along i, j or k) held in registers, as
+// its even and odd halves (line_eo).  With the full matrices and two outputs
+// at a time it waited on the latency of its multiply-add chains (n = 9 on
+// 3456 deformed elements: 63.6 us, now 47.3; n = 10 on 1728 affine 30.8, now
+// 26.6; n = 12 on 576 deformed 24.7, now 20.6).  Per element: the field is staged in shared memory; lines
 // along i and j give the r- and s-derivatives; the lines along k take the
 // t-derivative in registers, apply the six metric terms at their points and
 // form the t-transposed contribution S^T w2 in registers; lines along i and
 // j then turn w0 and w1 into D^T w0 and S^T w1 (D for Poisson) in place, and
 // the k-lines write the output (acc + acs) + act, the order of ax_element:
-// three staged fields and four block barriers per element group.  The matrices sit in shared memory and every lane of a warp
-// reads the same entry (a broadcast), two entries per paired load.  EPB
+// three staged fields and four block barriers per element group.  The
+// matrices sit in shared memory and every lane of a warp reads the same
+// entries (broadcasts of pairs).  AFF: a level of affine elements reads six
+// constants an element instead of six factors a point (Helmholtz at n = 12 on
+// 576 elements, fused: 36.7 us with the factors, 26.2 without).  EPB
 // elements per group fill about 256 threads.  The arithmetic runs in the
 // storage type T: FP64 for the solves, FP32 in the mixed-precision V-cycle
-// (the fused direction update and the p . (A p) sum stay FP64).  AFF: a
-// level of affine elements reads six constants an element instead of six
-// factors a point (Helmholtz at n = 12 on 576 elements, fused: 36.7 us with
-// the factors, 26.2 without; FP32 at n = 8 on 4096: 34.1 and 25.0).
+// (the fused direction update and the p . (A p) sum stay FP64).
 // ---------------------------------------------------------------------------
 template <int N>
 struct AxLine {
   static constexpr int EPB = (256 / (N * N)) > 0 ? 256 / (N * N) : 1;
   static constexpr int TASKS = EPB * N * N;
   static constexpr int THREADS = (TASKS + 31) / 32 * 32;
-  static constexpr int RM = N + (N & 1);                 // matrix rows (pair-aligned)
   static constexpr int RS = N + ((2 - N % 4) + 4) % 4;   // field rows: 2 mod 4 values
   static constexpr int FS = N * N * RS;                  // one staged field
-  static constexpr int MATS = 4 * N * RM;
+  static constexpr int MATS = 4 * EoMat<N>::SIZE;        // SIZE is even
   static constexpr int SMEM = MATS + EPB * 3 * FS;       // values of type T
 };
 
-// sum_l A[o][l] x[l] (A rows of RM values, pair-aligned), in l order; every
-// lane of the warp reads the same A entries
-template <int N, int RM, typename C>
-__device__ __forceinline__ C line_row(const C* A, int o, const C (&x)[N]) {
-  using V2 = typename std::conditional<sizeof(C) == 8, double2, float2>::type;
-  C acc = 0;
+// Blocks an SM the line-form kernel asks for: only where the compiler's own
+// choice of registers leaves too few warps (FP64: n = 9; from n = 10 the
+// Laplacian -- n = 12 unbounded takes 216 registers, five warps an SM: 26.7
+// us on 576 affine elements, 20.6 with two blocks; n = 10 35.0 and 26.6).
+// Elsewhere the bound makes it slower (n = 7: 15.1 -> 16.4, n = 5: 15.4 ->
+// 17.5, FP32 likewise).
+template <int N, typename T, bool HELM>
+constexpr int axl_blocks() {
+  if (sizeof(T) == 4 || N < 9 || (N >= 10 && HELM)) return 1;
+  return N == 11 ? 4 : 2;
+}
+
+// y = A x; every lane of the warp reads the same entries (broadcasts of
+// pairs), every output is its own chain of multiply-adds
+template <int N, typename T>
+__device__ __forceinline__ void line_eo(const T* A, const T (&x)[N], T (&y)[N]) {
+  using M = EoMat<N>;
+  using V2 = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+  constexpr int H = M::H, C = M::C;
+  T a[M::EP], b[M::OP > 0 ? M::OP : 1];
 #pragma unroll
-  for (int l = 0; l + 1 < N; l += 2) {
-    const V2 a = *reinterpret_cast<const V2*>(A + o * RM + l);
-    acc += a.x * x[l];
-    acc += a.y * x[l + 1];
+  for (int o = 0; o < M::EP; ++o) a[o] = 0;
+#pragma unroll
+  for (int o = 0; o < M::OP; ++o) b[o] = 0;
+#pragma unroll
+  for (int l = 0; l < C; ++l) {
+    const bool mid = l == H;   // (odd orders)
+    const T e = mid ? x[H] : x[l] + x[N - 1 - l], d = x[l] - x[N - 1 - l];
+    if (!mid)
+#pragma unroll
+      for (int o = 0; o < C; o += 2) {
+        const V2 m = *reinterpret_cast<const V2*>(A + l * M::EP + o);
+        a[o] += m.x * d;
+        if (o + 1 < C) a[o + 1] += m.y * d;
+      }
+#pragma unroll
+    for (int o = 0; o < H; o += 2) {
+      const V2 m = *reinterpret_cast<const V2*>(A + M::O0 + l * M::OP + o);
+      b[o] += m.x * e;
+      if (o + 1 < H) b[o + 1] += m.y * e;
+    }
   }
-  if (N & 1) acc += A[o * RM + N - 1] * x[N - 1];
-  return acc;
+#pragma unroll
+  for (int o = 0; o < H; ++o) {
+    y[o] = a[o] + b[o];
+    y[N - 1 - o] = a[o] - b[o];
+  }
+  if (N & 1) y[H] = a[H];
 }
 
-// dst[o * stride] (=, or += when ADD) sum_l A[o][l] x[l] for o < N; the
-// output loop is not unrolled, so a line's matrix rows are read one row at
-// a time and the registers hold the line only
-template <int N, int RM, bool ADD, typename C>
-__device__ __forceinline__ void line_apply(const C* A, const C (&x)[N], C* dst, int stride) {
-#pragma unroll 2
-  for (int o = 0; o < N; ++o) {
-    const C v = line_row<N, RM, C>(A, o, x);
-    if (ADD)
-      dst[o * stride] += v;
-    else
-      dst[o * stride] = v;
+// the halves of G (N x N, or its transpose) into shared memory; the two
+// entries that the symmetry makes equal are averaged
+template <int N, typename T>
+__device__ __forceinline__ void eo_load(T* A, const double* __restrict__ G, bool transposed) {
+  using M = EoMat<N>;
+  auto at = [&](int o, int l) {
+    const double p = transposed ? G[l * N + o] : G[o * N + l];
+    const double q = transposed ? G[(N - 1 - l) * N + N - 1 - o] : G[(N - 1 - o) * N + N - 1 - l];
+    return 0.5 * (p - q);
+  };
+  for (int q = threadIdx.x; q < M::SIZE; q += blockDim.x) {
+    double v = 0.0;
+    if (q < M::O0) {
+      const int l = q / M::EP, o = q % M::EP;
+      if (o < M::C) v = 0.5 * (at(o, l) - at(o, N - 1 - l));
+    } else {
+      const int l = (q - M::O0) / M::OP, o = (q - M::O0) % M::OP;
+      if (o < M::H) v = l == M::H ? at(o, l) : 0.5 * (at(o, l) + at(o, N - 1 - l));
+    }
+    A[q] = (T)v;
   }
 }
 
-// D, D^T, S (Helmholtz) or D, S^T = D^T into the first MATS values of the
-// block's shared memory; visible after the next barrier
+// D, D^T, S, S^T (Poisson: D, D^T only, in the same places) into the first
+// MATS values of the block's shared memory; visible after the next barrier
 template <int N, typename T, bool HELM>
 __device__ __forceinline__ void axl_load_mats(T* sD, const double* __restrict__ Dg,
                                               const double* __restrict__ Sg) {
-  constexpr int RM = AxLine<N>::RM;
-  T* sDT = sD + N * RM;
-  T* sS = sDT + N * RM;
-  T* sST = sS + N * RM;
-  for (int q = threadIdx.x; q < N * N; q += blockDim.x) {
-    const int r = q / N, c = q % N;
-    const T d = (T)Dg[q], sv = HELM ? (T)Sg[q] : d;
-    sD[r * RM + c] = d;
-    sDT[c * RM + r] = d;
-    sS[r * RM + c] = sv;
-    sST[c * RM + r] = sv;
+  constexpr int E = EoMat<N>::SIZE;
+  eo_load<N, T>(sD, Dg, false);
+  eo_load<N, T>(sD + E, Dg, true);
+  if (HELM) {
+    eo_load<N, T>(sD + 2 * E, Sg, false);
+    eo_load<N, T>(sD + 3 * E, Sg, true);
   }
 }
 
@@ -642,10 +692,10 @@ __device__ __forceinline__ double axl_group(int e0, int ne, T* __restrict__ u,
                                             const AffGeom& ag) {
   using L = AxLine<N>;
   using C = T;
-  constexpr int NN = N * N, NT = N * N * N, RM = L::RM, RS = L::RS, FS = L::FS;
-  const C* sDT = sD + N * RM;
-  const C* sS = sDT + N * RM;
-  const C* sST = sS + N * RM;
+  constexpr int NN = N * N, NT = N * N * N, RS = L::RS, FS = L::FS, ES = EoMat<N>::SIZE;
+  const C* sDT = sD + ES;
+  const C* sS = HELM ? sD + 2 * ES : sD;
+  const C* sST = HELM ? sD + 3 * ES : sDT;
   C* fld = sD + L::MATS;   // per slot: U, F1, F2 (FS values each)
   const int tid = threadIdx.x;
   const size_t base = (size_t)e0 * NT;
@@ -686,18 +736,24 @@ __device__ __forceinline__ double axl_group(int e0, int ne, T* __restrict__ u,
   C* F2 = F1 + FS;
   // P1, P2: derivatives along i (r, with S for Helmholtz) and j (s)
   if (task) {
-    C x[N];
+    C x[N], y[N];
     {   // lines (j = a0, k = a1) along i
       const C* src = U + a1 * N * RS + a0 * RS;
 #pragma unroll
       for (int l = 0; l < N; ++l) x[l] = src[l];
-      line_apply<N, RM, false, C>(HELM ? sS : sD, x, F1 + a1 * N * RS + a0 * RS, 1);
+      line_eo<N, C>(sS, x, y);
+      C* dst = F1 + a1 * N * RS + a0 * RS;
+#pragma unroll
+      for (int l = 0; l < N; ++l) dst[l] = y[l];
     }
     {   // lines (i = a0, k = a1) along j
       const C* src = U + a1 * N * RS + a0;
 #pragma unroll
       for (int l = 0; l < N; ++l) x[l] = src[l * RS];
-      line_apply<N, RM, false, C>(sD, x, F2 + a1 * N * RS + a0, RS);
+      line_eo<N, C>(sD, x, y);
+      C* dst = F2 + a1 * N * RS + a0;
+#pragma unroll
+      for (int l = 0; l < N; ++l) dst[l * RS] = y[l];
     }
   }
   __syncthreads();
@@ -708,10 +764,11 @@ __device__ __forceinline__ double axl_group(int e0, int ne, T* __restrict__ u,
   C act[N];
   const size_t eo = base + (size_t)sl * NT + a1 * N + a0;
   if (task) {
-    C x[N], w2[N];
+    C x[N], ut[N];
     const C* src = U + a1 * RS + a0;
 #pragma unroll
     for (int l = 0; l < N; ++l) x[l] = src[l * N * RS];
+    line_eo<N, C>(sD, x, ut);
     // affine: the element's constant metric, the weights of this line
     C cg[6];
     double wij = 0.0;
@@ -720,9 +777,8 @@ __device__ __forceinline__ double axl_group(int e0, int ne, T* __restrict__ u,
       for (int a = 0; a < 6; ++a) cg[a] = (C)__ldg(ag.c + 6 * (size_t)(e0 + sl) + a);
       wij = __ldg(ag.w + a0) * __ldg(ag.w + a1);
     }
-#pragma unroll 2
+#pragma unroll
     for (int k = 0; k < N; ++k) {
-      const C ut = line_row<N, RM, C>(sD, k, x);
       const int q = k * N * RS + a1 * RS + a0;
       const size_t o = eo + (size_t)k * NN;
       const C ur = F1[q], us = F2[q];
@@ -739,30 +795,33 @@ __device__ __forceinline__ double axl_group(int e0, int ne, T* __restrict__ u,
         g4 = __ldg(gf + 4 * npts + o);
         g5 = __ldg(gf + 5 * npts + o);
       }
-      F1[q] = g0 * ur + g1 * us + g2 * ut;
-      F2[q] = g1 * ur + g3 * us + g4 * ut;
-      w2[k] = g2 * ur + g4 * us + g5 * ut;
+      F1[q] = g0 * ur + g1 * us + g2 * ut[k];
+      F2[q] = g1 * ur + g3 * us + g4 * ut[k];
+      x[k] = g2 * ur + g4 * us + g5 * ut[k];
     }
-#pragma unroll
-    for (int k = 0; k < N; ++k) act[k] = line_row<N, RM, C>(sST, k, w2);
+    line_eo<N, C>(sST, x, act);
   }
   __syncthreads();
   // P4: the r-transposed D^T w0 along i and the s-transposed S^T w1 along
   // j, each written over its own input line (a thread reads the whole line
   // before it writes it)
   if (task) {
-    C x[N];
+    C x[N], y[N];
     {   // lines (j = a0, k = a1) along i
       C* line = F1 + a1 * N * RS + a0 * RS;
 #pragma unroll
       for (int l = 0; l < N; ++l) x[l] = line[l];
-      line_apply<N, RM, false, C>(sDT, x, line, 1);
+      line_eo<N, C>(sDT, x, y);
+#pragma unroll
+      for (int l = 0; l < N; ++l) line[l] = y[l];
     }
     {   // lines (i = a0, k = a1) along j
       C* line = F2 + a1 * N * RS + a0;
 #pragma unroll
       for (int l = 0; l < N; ++l) x[l] = line[l * RS];
-      line_apply<N, RM, false, C>(sST, x, line, RS);
+      line_eo<N, C>(sST, x, y);
+#pragma unroll
+      for (int l = 0; l < N; ++l) line[l * RS] = y[l];
     }
   }
   __syncthreads();

@@ -312,16 +312,16 @@ ssg_status run_request(ssg_server* S, Request* r, Resident* slot) {
 struct BatchArena {
   ssg_context* c = nullptr;
   ssg::SegScratch W;
-  double *gf = nullptr, *bj = nullptr, *kdiag = nullptr, *det = nullptr;
+  double *gf = nullptr, *bj = nullptr, *kdiag = nullptr, *det = nullptr, *aff = nullptr;
   uint8_t* mult = nullptr;
   int* dss = nullptr;
   size_t cap_points = 0, cap_dss = 0;
   void release() {
     ssg::seg_scratch_free(W);
-    void* ps[] = {gf, bj, kdiag, det, mult, dss};
+    void* ps[] = {gf, bj, kdiag, det, aff, mult, dss};
     for (void* p : ps)
       if (p) cudaFree(p);
-    gf = bj = kdiag = det = nullptr;
+    gf = bj = kdiag = det = aff = nullptr;
     mult = nullptr;
     dss = nullptr;
     cap_points = cap_dss = 0;
@@ -373,6 +373,7 @@ ssg_status run_batch(ssg_server* S, BatchArena& A, std::vector<Request*>& b,
     SSG_TRY(arena_alloc(c, &A.kdiag, cap));
     SSG_TRY(arena_alloc(c, &A.det, cap));
     SSG_TRY(arena_alloc(c, &A.mult, cap));
+    SSG_TRY(arena_alloc(c, &A.aff, cap / 8 * 6));
     A.cap_points = cap;
   }
   if (ndss > A.cap_dss) {
@@ -384,10 +385,20 @@ ssg_status run_batch(ssg_server* S, BatchArena& A, std::vector<Request*>& b,
     A.cap_dss = cap;
   }
   cudaStream_t s = c->stream;
+  // all affine: six constants an element in place of the per-point factors
+  bool aff = true, sym = true;
+  for (Resident* r : sl) {
+    aff = aff && r->ctx->lev[0].aff;
+    sym = sym && r->ctx->lev[0].sym;
+  }
   for (size_t k = 0; k < b.size(); ++k) {
     const ssg::DevLevel& D = sl[k]->ctx->lev[0];
     const size_t P = (size_t)first[k] * nt, m = D.npts;
-    for (int a = 0; a < 6; ++a)
+    if (aff)
+      SSG_CUDA(c, cudaMemcpyAsync(A.aff + 6 * (size_t)first[k], D.aff,
+                                  6 * (size_t)b[k]->d.nel * sizeof(double),
+                                  cudaMemcpyDeviceToDevice, s));
+    for (int a = 0; a < 6 && !aff; ++a)
       SSG_CUDA(c, cudaMemcpyAsync(A.gf + a * np + P, D.gf + a * m, m * sizeof(double),
                                   cudaMemcpyDeviceToDevice, s));
     SSG_CUDA(c, cudaMemcpyAsync(A.bj + P, D.bj, m * sizeof(double), cudaMemcpyDeviceToDevice, s));
@@ -414,6 +425,9 @@ ssg_status run_batch(ssg_server* S, BatchArena& A, std::vector<Request*>& b,
   L.S = D0.S;
   L.mult = A.mult;
   L.dss = A.dss;
+  L.ag = ssg::aff_geom(D0);
+  L.ag.c = aff ? A.aff : nullptr;
+  L.ag.sym = sym;
   std::vector<double> u(np, 0.0);
   std::vector<ssg_solve_info> info(b.size());
   int max_iter = 0;

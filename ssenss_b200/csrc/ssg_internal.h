@@ -117,6 +117,7 @@ struct DevLevel {
   double* bj = nullptr;        // rho * J
   double* aff = nullptr;       // nel x 6: G_ab J where every element is affine, else null
   double* w = nullptr;         // n GLL weights (with aff)
+  bool sym = false;            // D and S antisymmetric under index reversal
   double* kdiag = nullptr;     // element-local stiffness diagonal
   double* dinv_p = nullptr;    // Poisson Jacobi inverse
   double* dinv_h = nullptr;    // Helmholtz Jacobi inverse (for lambda_h)
@@ -139,6 +140,7 @@ inline AffGeom aff_geom(const DevLevel& L) {
   AffGeom a;
   a.c = L.aff;
   a.w = L.w;
+  a.sym = L.sym;
   return a;
 }
 
@@ -155,6 +157,7 @@ struct SegLevel {
   const double *mask = nullptr, *D = nullptr, *S = nullptr;
   const uint8_t* mult = nullptr;
   const int* dss = nullptr;    // DSS map (dss_map_table layout)
+  AffGeom ag;                  // the level's constant metric and matrix symmetry
 };
 
 // Device scratch of segmented solves, grown on demand and reused.

@@ -94,6 +94,9 @@ struct PUpdateArgs {
 struct AffGeom {
   const double* c = nullptr;
   const double* w = nullptr;   // n GLL weights
+  // the level's D and S are antisymmetric under reversal of both indices (the
+  // line-form kernel's even / odd split; without it the plane form runs)
+  bool sym = false;
 };
 
 // kernel launches of this library: process-wide, and per host thread (the
@@ -134,7 +137,7 @@ int vec_blocks(size_t npts);
 // than 8; 1, 2, 4, ... select the plane-form kernel k_ax with that many
 // elements per block; 0 asks for the order's default (ax_epb)
 constexpr int kAxLine = -1;
-int ax_epb(int n);
+int ax_epb(int n, bool sym);
 int ax_epb_max(int n);
 int dss_grid(int n, int nel);
 // autotuned launch shapes (0 = default rule), indexed by order n; atomics:

@@ -51,12 +51,14 @@ static ssg_status tune_level(ssg_context* c, int level, double* a, double* b, do
                              int reps) {
   const DevLevel& L = c->lev[level];
   const int n = L.n;
-  // operator: elements per block (order 8 has the tensor-core kernel only)
-  if (n != 8) {
+  // operator: the line form where the level's matrices have the points'
+  // symmetry (its even / odd split beats every plane form at every order and
+  // rounds differently, so it is not a matter of timing); else the plane
+  // form's elements per block (order 8 has the tensor-core kernel only)
+  if (n != 8 && !L.sym) {
     int best_epb = 0;
     float best = 1e30f;
-    for (int epb = kAxLine; epb <= ax_epb_max(n); epb = epb == kAxLine ? 1 : 2 * epb) {
-      g_tune_ax_epb[n] = epb;
+    for (int epb = 1; epb <= ax_epb_max(n); epb *= 2) {
       SSG_CUDA(c, run_ax(c->stream, n, c->nel, epb, false, false, a, b, L.gf, L.npts, nullptr,
                          L.D, L.D, 0.0, nullptr, aff_geom(L)));
       float t = 0.f;
@@ -243,7 +245,7 @@ ssg_status ssg_tuning(int n, int* ax_elements_per_block, int* dss_blocks_per_sm,
   if (n < 2 || n > SSG_MAXN) return SSG_ERR_ARG;
   // 0: the FP64 tensor-core operator (one warp per element)
   const bool dmma = n == 8;
-  if (ax_elements_per_block) *ax_elements_per_block = dmma ? 0 : ax_epb(n);
+  if (ax_elements_per_block) *ax_elements_per_block = dmma ? 0 : ax_epb(n, true);
   if (dss_blocks_per_sm) *dss_blocks_per_sm = g_tune_dss_bps[n].load() > 0 ? g_tune_dss_bps[n].load() : 8;
   if (vector_blocks_per_sm) *vector_blocks_per_sm = g_tune_vec_bps.load() > 0 ? g_tune_vec_bps.load() : kVecBpsDefault;
   return SSG_OK;

@@ -155,3 +155,36 @@ def test_convection_with_matrices_that_are_not_symmetric(n, gpu_ctx_factory):
     assert rel(ctx.convection_operator(u, v), conv_reference(u, v, J, D, w, det, tinv)) < 1e-13
     ctx.close()
     orc.close()
+
+
+@pytest.mark.parametrize("n", [3, 6, 7])
+def test_operator_with_a_matrix_that_is_not_antisymmetric(n, gpu_ctx_factory):
+    """A caller's own derivative matrix without the points' symmetry, through
+    the drop-in set-up: the line kernel's even / odd split does not apply, the
+    result is the definition's all the same (1e-13)."""
+    import ssenss_b200 as S
+    m = box_mesh((3, 3, 3))
+    orc = O.Oracle(m, n)
+    rng = np.random.default_rng(n)
+    ctx = S.Context(0)
+    ctx.setup_connectivity(m.neigh)
+    for level, nl in enumerate(orc.orders):
+        D = rng.standard_normal((nl, nl))
+        w = rng.uniform(0.1, 1.0, nl)
+        geom = rng.uniform(0.5, 1.5, (6, m.nel, nl, nl, nl))
+        det = rng.uniform(0.5, 1.5, (m.nel, nl, nl, nl))
+        interp = None if level == 0 else rng.standard_normal((nl, orc.orders[level - 1]))
+        ctx.setup_level(level, nl, np.ascontiguousarray(D.T), None, w, geom, det, interp)
+        if level == 0:
+            D0, w0, g0, d0 = D, w, geom, det
+    ctx.setup_finish()
+    u = rng.standard_normal((m.nel, n, n, n))
+    ax = ("pi,ekji->ekjp", "pj,ekji->ekpi", "pk,ekji->epji")
+    du = [np.einsum(ax[b], D0, u) for b in range(3)]
+    rho = (w0[:, None, None] * w0[:, None] * w0) * d0
+    sym = [[0, 1, 2], [1, 3, 4], [2, 4, 5]]
+    ref = sum(np.einsum(ax[a], D0.T, sum(g0[sym[a][b]] * du[b] for b in range(3)) * rho)
+              for a in range(3))
+    assert rel(ctx.local_opeval(O.PRESSURE, u), ref) < 1e-13
+    ctx.close()
+    orc.close()
