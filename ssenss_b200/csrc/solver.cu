@@ -362,14 +362,14 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
   // all of them for a smoother (sync_each false), chunks of 8 otherwise.
   const double* stop = fr + F_DONE;
   pu.stop = stop;
-  // Mixed precision (FP32 storage): (p w).DSS(mask A p) = p . (mask A p)
-  // for a continuous, masked p, so the operator kernel reduces it, alpha is
-  // known before the DSS, and the DSS gather feeds the update directly (two
-  // kernels per iteration, ap never stored).  FP64 keeps the reference's
-  // arithmetic: alpha from the weighted dot of the assembled ap
-  // (src/solver.c:62-65), then the update -- the rounding of the fused form
-  // moves a well-converged solution by a few 1e-11.
-  const bool fused = fp32;
+  // (p w).DSS(mask A p) = p . (mask A p) for a continuous, masked p, so the
+  // operator kernel reduces it, alpha is known before the DSS, and the DSS
+  // gather feeds the update directly: two kernels per iteration, ap never
+  // stored (FP64 on the periodic 16^3 box at n = 8: 15.6 + 28.4 us for the DSS
+  // and the update apart; the solve 24.7 -> 22.6 ms fused).  On meshes
+  // without the line-run DSS (irregular pairing) the FP64 gather and update
+  // stay apart, as the gather-word kernel gains nothing fused (62 us).
+  const bool fused = fp32 || c->d_nbreg;
   ScalarOp dop = op;
   if (fused) {
     pu.dot = &dop;
