@@ -51,7 +51,12 @@ static ssg_status dupload(ssg_context* c, T** p, const T* src, size_t count) {
 }
 
 static ssg_status upload_f32(ssg_context* c, float** p, const double* src, size_t count) {
-  std::vector<float> t(src, src + count);
+  std::vector<float> t(count);
+  const size_t blk = 1 << 14;   // converted on all host threads
+  parallel_elements((int)((count + blk - 1) / blk), [&](int b0, int b1) {
+    const size_t hi = std::min(count, (size_t)b1 * blk);
+    for (size_t q = (size_t)b0 * blk; q < hi; ++q) t[q] = (float)src[q];
+  });
   return dupload(c, p, t.data(), count);
 }
 
@@ -259,10 +264,16 @@ static ssg_status upload_all(ssg_context* c) {
     stiffness_diagonal(h, nel, kd.data());
     std::vector<double> dp(kd);
     host_dss(H, h.n, dp.data());
-    for (auto& v : dp) v = 1.0 / v;
     std::vector<double> sc(np, 1.0);
     host_dss(H, h.n, sc.data());
-    for (auto& v : sc) v = 1.0 / v;
+    std::vector<uint8_t> mu(np);
+    parallel_elements(nel, [&](int e0, int e1) {
+      for (size_t q = e0 * h.nt; q < (size_t)e1 * h.nt; ++q) {
+        dp[q] = 1.0 / dp[q];
+        mu[q] = (uint8_t)std::lround(sc[q]);
+        sc[q] = 1.0 / sc[q];
+      }
+    });
     double nun = 0.0;
     for (double v : sc) nun += v;
     d.nunique = nun;
@@ -295,11 +306,7 @@ static ssg_status upload_all(ssg_context* c) {
     SSG_TRY(dupload(c, &d.dinv_p, dp.data(), np));
     SSG_TRY(dalloc(c, &d.dinv_h, np));
     d.lambda_h = -1.0;
-    {
-      std::vector<uint8_t> mu(np);
-      for (size_t q = 0; q < np; ++q) mu[q] = (uint8_t)std::lround(1.0 / sc[q]);
-      SSG_TRY(dupload(c, &d.mult, mu.data(), np));
-    }
+    SSG_TRY(dupload(c, &d.mult, mu.data(), np));
     if (c->has_walls) {
       std::vector<double> mk(np, 1.0);
       const int n = h.n;
