@@ -459,28 +459,36 @@ void dss_map_table(const HostMesh& m, int n, std::vector<int>& tab) {
 
 // The factors of an affine element are one constant up to the rounding of
 // the differentiated node coordinates, relative noise of about eps |x| n^2 / h
-// (measured on boxes of 3 to 32 elements along a side: 3e-14 at n = 6, 1e-12
-// at n = 8, 2e-12 at n = 10 and 12), so a level counts as affine when no
-// factor is further than affine_noise(n) of the element's largest one from
-// the element's mean.  A deformation of the mesh shows in the factors at its
-// own relative size.  The mean is closer to the exact constant than the
-// single values are (5e-14 against 1e-12 on the periodic 16^3 box at n = 8).
-// Not affine: any element outside the bound, a factor that is not finite.
-// Means within the bound of zero are zero (the off-diagonal terms of an
-// axis-aligned element).
+// (measured on boxes of 3 to 32 elements along a side: 4e-14 at n = 6, 1e-12
+// at n = 8 and 3e-12 at n = 12, on dealiasing grids 3e-12 at m = 12 and 1e-11
+// at m = 18), so a level counts as affine when no factor is further than
+// affine_noise(n) of its own natural size from the element's mean.  The
+// natural size of G_ab is sqrt(G_aa G_bb): on thin elements the factors differ
+// by the aspect ratio squared, and each has to be constant on its own scale
+// (measured against the largest, a 1 x 1e-6 x 1 element lost G_11 and G_33,
+// and a twist of 1e-9 of sqrt(G_11 G_22) at aspect 1000 passed as noise).  A
+// deformation of the mesh shows in the factors at its own relative size.  The
+// rounding of the cross terms grows with |x| / h of the thin direction and
+// passes the bound from aspect ratios of some tens on: such levels keep the
+// per-point factors.  The mean is closer to the exact constant than the single
+// values are (5e-14 against 1e-12 on the periodic 16^3 box at n = 8).
+// Not affine: any element outside the bound, a factor that is not finite, a
+// zero natural size.  Cross terms whose mean is within the bound of zero are
+// zero (axis-aligned elements).
 static double affine_noise(int n) { return 4e-14 * n * n; }
 
-// nf factors f[a] (times det when given) of nel elements of nt points: their
-// means, nf per element, or empty
+// nf factors f[a] times det of nel elements of nt points: their means, nf per
+// element, or empty.  size(mean, a): the natural size of factor a.
+template <class Size>
 static void element_constants(int n, int nel, size_t nt, int nf, const double* const* f,
-                              const double* det, std::vector<double>& c) {
+                              const double* det, Size&& size, std::vector<double>& c) {
   c.assign((size_t)nel * nf, 0.0);
   const double noise = affine_noise(n);
   std::atomic<bool> affine{true};
   parallel_elements(nel, [&](int e0, int e1) {
     for (int e = e0; e < e1 && affine.load(std::memory_order_relaxed); ++e) {
       const size_t o = (size_t)e * nt;
-      double mean[9], lo[9], hi[9], top = 0.0;
+      double mean[9], lo[9], hi[9];
       for (int a = 0; a < nf; ++a) {
         double s = 0.0, mn = f[a][o] * det[o], mx = mn;
         for (size_t q = 0; q < nt; ++q) {
@@ -492,16 +500,16 @@ static void element_constants(int n, int nel, size_t nt, int nf, const double* c
         mean[a] = s / (double)nt;
         lo[a] = mn;
         hi[a] = mx;
-        top = std::max(top, std::fabs(mean[a]));
       }
-      // (a NaN among the factors makes its mean, and top or the test, NaN)
-      const double tol = noise * top;
-      bool ok = std::isfinite(top) && top > 0.0;
-      for (int a = 0; a < nf; ++a)
-        ok = ok && hi[a] - mean[a] <= tol && mean[a] - lo[a] <= tol;
-      if (!ok) affine.store(false, std::memory_order_relaxed);
-      for (int a = 0; a < nf; ++a)
+      // (a NaN among the factors makes its mean and so the tests fail)
+      bool ok = true;
+      for (int a = 0; a < nf; ++a) {
+        const double top = size(mean, a), tol = noise * top;
+        ok = ok && std::isfinite(top) && top > 0.0 && hi[a] - mean[a] <= tol &&
+             mean[a] - lo[a] <= tol;
         c[(size_t)nf * e + a] = std::fabs(mean[a]) <= tol ? 0.0 : mean[a];
+      }
+      if (!ok) affine.store(false, std::memory_order_relaxed);
     }
   });
   if (!affine.load()) c.clear();
@@ -510,14 +518,27 @@ static void element_constants(int n, int nel, size_t nt, int nf, const double* c
 void affine_metric(const HostLevel& L, int nel, std::vector<double>& c) {
   const double* g[6];
   for (int a = 0; a < 6; ++a) g[a] = L.g[a].data();
-  element_constants(L.n, nel, L.nt, 6, g, L.det.data(), c);
+  // G11 G12 G13 G22 G23 G33: the diagonal terms of each factor's indices
+  static const int da[6] = {0, 0, 0, 3, 3, 5}, db[6] = {0, 3, 5, 3, 5, 5};
+  element_constants(L.n, nel, L.nt, 6, g, L.det.data(),
+                    [](const double* m, int a) {
+                      return std::sqrt(std::fabs(m[da[a]])) * std::sqrt(std::fabs(m[db[a]]));
+                    },
+                    c);
 }
 
 void affine_convection(const HostLevel& L, int nel, std::vector<double>& c) {
   const double* t[9];
   for (int b = 0; b < 3; ++b)
     for (int a = 0; a < 3; ++a) t[3 * b + a] = L.tinv[3 * a + b].data();
-  element_constants(L.n, nel, L.nt, 9, t, L.det.data(), c);
+  // natural size: the largest weight of the reference direction b
+  element_constants(L.n, nel, L.nt, 9, t, L.det.data(),
+                    [](const double* m, int a) {
+                      const double* r = m + a / 3 * 3;
+                      return std::max(std::fabs(r[0]),
+                                      std::max(std::fabs(r[1]), std::fabs(r[2])));
+                    },
+                    c);
   for (auto& v : c) v *= 0.5;
 }
 
