@@ -337,7 +337,14 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
     // (n = 8 keeps its FP64 factors in fragment order: affine levels only)
     if (max_iter > 0 && (R.gf || R.ag.c))
       SSG_CUDA(c, run_cluster_cg(s, c->device, L.n, fp32, R, true, &fits));
-    if (fits) return sync_each ? cg_outcome(c, fr, eps, max_iter) : SSG_OK;
+    if (fits) {
+      if (!sync_each) return SSG_OK;
+      // (the flag and the deadline count once the kernel has ended, as after
+      // the loop graph below)
+      SSG_CUDA(c, cudaStreamSynchronize(s));
+      SSG_TRY(check_interrupt(c));
+      return cg_outcome(c, fr, eps, max_iter);
+    }
   }
 
   // mask f; r = f - A x; subtract_nullspace(r)
