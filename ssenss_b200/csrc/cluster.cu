@@ -8,16 +8,20 @@
 // 17.8 us an iteration, and as one cooperative launch with three grid-wide
 // barriers the n = 4 level under it takes 14.8 us, for 4,096 points.  In a
 // cluster a barrier is a hardware barrier over at most 16 SMs, a neighbour
-// element's copy of a node is one distributed-shared-memory load, and the
-// two sums of an iteration travel as one value per SM.
+// element's copy of a node is one load from L2 (the exchanged vector is the
+// only one in global memory: gathered from distributed shared memory, a warp's
+// scattered loads took 15 cycles each), and the sums of an iteration travel
+// as one value per SM through distributed shared memory.
 //
 // Arithmetic: conjugate_gradient with jacobi_preconditioner
 // (src/solver.c:33-81, src/precon.c:311-324) as cg_solve's kernels do it --
 // the same rounding to the storage type T, the DSS in the reference's order,
-// FP64 sums -- except that p.(A p) is summed over the element copies before
-// the DSS (equal to the weighted product for a continuous p), so that it is
-// known at the same barrier as the operator's output.  Every block adds the
-// blocks' partial sums in rank order, so all take the same alpha, beta and
+// FP64 sums -- except that where p is the same in all copies of a node (the
+// levels below level 0; FP32 as in its kernels) p.(A p) is summed over the
+// element copies before the DSS, equal to the weighted product, so that it is
+// known at the same barrier as the operator's output; the FP64 solve of level
+// 0 takes (p w).ap of the assembled ap and one more barrier.  Every block adds
+// the blocks' partial sums in rank order, so all take the same alpha, beta and
 // stop decision.
 #include <cuda_runtime.h>
 
@@ -134,6 +138,7 @@ struct ClusterCgArgs {
   const int* dss = nullptr;       // DSS map (dss_map_table)
   AffGeom ag;
   int helm = 0, pressure = 0;
+  int weighted = 0;               // alpha from the assembled A p
   int sgeom = 0;                  // per-point factors in shared memory
   double nunique = 1.0, eps = 0.0;
   int max_iter = 0;
@@ -488,6 +493,21 @@ __global__ void __launch_bounds__(512) k_cluster_cg(ClusterCgArgs<T> a) {
     });
     __syncthreads();
     d[0] = op();
+    if (a.weighted) {
+      // (p w).ap of the assembled ap: one more barrier
+      cluster_sync();
+      dss();
+      d[0] = 0.0;
+      points([&](const int (&q)[4], const int (&o)[4], const bool (&ok)[4]) {
+        double pa[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          pa[h] = ((double)U[o[h]] * inv_count(MU[q[h]])) * (double)F2[o[h]];
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          if (ok[h]) d[0] += pa[h];
+      });
+    }
     if (first) {
       red_post<3>(red, buf, d, cs, rank);
     } else {
@@ -495,7 +515,7 @@ __global__ void __launch_bounds__(512) k_cluster_cg(ClusterCgArgs<T> a) {
       red_post<1>(red, buf, s, cs, rank);
     }
     cluster_sync();
-    dss();
+    if (!a.weighted) dss();
     if (first) {
       red_sum<3>(red, buf, cs, d);
       rdz = d[1];
@@ -922,6 +942,7 @@ cudaError_t cluster_cg_n(cudaStream_t s, int device, const ClusterCgRun& L, bool
   a.ag = L.ag;
   a.helm = L.helm;
   a.pressure = !L.helm;
+  a.weighted = L.weighted;
   a.sgeom = sgeom;
   a.nunique = L.nunique;
   a.eps = L.eps;

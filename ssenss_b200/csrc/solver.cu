@@ -279,6 +279,15 @@ static ssg_status cg_outcome(ssg_context* c, const double* fr, double eps, int m
   return SSG_OK;
 }
 
+// Whether all copies of a node hold the same p in the CG of a level.  Below
+// level 0 the right-hand side is a DSS average and the start a prolonged
+// continuous field.  At level 0 the caller's right-hand side may differ
+// between copies, and where a wall meets an element in an edge alone the
+// element's copies of that edge are not masked: the FP64 solve there keeps the
+// reference's alpha, from the weighted dot of the assembled ap
+// (src/solver.c:62-65), for any input.
+static bool continuous_p(int level) { return level > 0; }
+
 ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void* x,
                     double eps, int max_iter, int frame, double* hist, int hist_cap,
                     bool sync_each) {
@@ -333,6 +342,7 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
     R.frame = fr;
     R.hist = hist;
     R.hist_cap = hist_cap;
+    R.weighted = !fp32 && !continuous_p(level);
     bool fits = false;
     // (n = 8 keeps its FP64 factors in fragment order: affine levels only)
     if (max_iter > 0 && (R.gf || R.ag.c))
@@ -369,14 +379,16 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
   // all of them for a smoother (sync_each false), chunks of 8 otherwise.
   const double* stop = fr + F_DONE;
   pu.stop = stop;
-  // (p w).DSS(mask A p) = p . (mask A p) for a continuous, masked p, so the
-  // operator kernel reduces it, alpha is known before the DSS, and the DSS
-  // gather feeds the update directly: two kernels per iteration, ap never
-  // stored (FP64 on the periodic 16^3 box at n = 8: 15.6 + 28.4 us for the DSS
-  // and the update apart; the solve 24.7 -> 22.6 ms fused).  On meshes
-  // without the line-run DSS (irregular pairing) the FP64 gather and update
-  // stay apart, as the gather-word kernel gains nothing fused (62 us).
-  const bool fused = fp32 || c->d_nbreg;
+  // (p w).DSS(mask A p) = p . (mask A p) when all copies of a node hold the
+  // same p, so the operator kernel reduces it, alpha is known before the DSS,
+  // and the DSS gather feeds the update directly: two kernels per iteration,
+  // ap never stored.  In FP64 only where p is continuous by construction
+  // (continuous_p; Poisson solves on periodic boxes, n = 12 on 10^3 elements
+  // 19.7 -> 19.1 ms, n = 9 on 14^3 24.2 -> 23.4; level 0 in this form as well
+  // would give 18.2 and 23.7, n = 8 on 16^3 21.2 for 23.0); on meshes without
+  // the line-run DSS (irregular pairing) the FP64 gather and update stay
+  // apart, as the gather-word kernel gains nothing fused (62 us).
+  const bool fused = fp32 || (c->d_nbreg && continuous_p(level));
   ScalarOp dop = op;
   if (fused) {
     pu.dot = &dop;

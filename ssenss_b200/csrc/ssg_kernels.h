@@ -240,6 +240,7 @@ struct ClusterCgRun {
   const double* mask = nullptr;
   const int* dss = nullptr;   // DSS map (dss_map_table)
   AffGeom ag;
+  int weighted = 0;           // alpha from (p w).DSS(A p): p may differ between copies
   double nunique = 1.0, eps = 0.0;
   int max_iter = 0;
   double* frame = nullptr;
