@@ -197,7 +197,8 @@ __global__ void __launch_bounds__(512) k_cluster_cg(ClusterCgArgs<T> a) {
   const uint32_t rank = cluster_rank();
   const int cs = a.cs, epc = a.epc;
   const int e0 = (int)rank * epc, ne = max(0, min(epc, a.nel - e0));
-  const bool aff = a.ag.c != nullptr;
+  // (FP32 reads its stored factors, each one rounding of the FP64 value)
+  const bool aff = sizeof(T) == 8 && a.ag.c != nullptr;
   T* const sD = reinterpret_cast<T*>(smem_raw);
   T* const sDT = sD + N * RM;
   T* const sS = sDT + N * RM;
@@ -918,7 +919,7 @@ cudaError_t cluster_cg_n(cudaStream_t s, int device, const ClusterCgRun& L, bool
   if (e != cudaSuccess) return e;
   int epc = 0;
   bool sgeom = false;
-  const bool aff = L.ag.c != nullptr;
+  const bool aff = sizeof(T) == 8 && L.ag.c;
   const int cs = cluster_blocks<N, T>(L.nel, most, aff, &epc, &sgeom);
   *fits = cs > 0;
   if (!cs || !launch) return cudaSuccess;

@@ -574,7 +574,9 @@ struct EoMat {
 // 576 elements, fused: 36.7 us with the factors, 26.2 without).  EPB
 // elements per group fill about 256 threads.  The arithmetic runs in the
 // storage type T: FP64 for the solves, FP32 in the mixed-precision V-cycle
-// (the fused direction update and the p . (A p) sum stay FP64).
+// (the fused direction update and the p . (A p) sum stay FP64, and a factor of
+// an affine element is one rounding of its FP64 value, as the stored ones are:
+// the FP32 products instead would save 1 % of a mixed solve).
 // ---------------------------------------------------------------------------
 template <int N>
 struct AxLine {
@@ -770,11 +772,10 @@ __device__ __forceinline__ double axl_group(int e0, int ne, T* __restrict__ u,
     for (int l = 0; l < N; ++l) x[l] = src[l * N * RS];
     line_eo<N, C>(sD, x, ut);
     // affine: the element's constant metric, the weights of this line
-    C cg[6];
-    double wij = 0.0;
+    double cg[6], wij = 0.0;
     if (AFF) {
 #pragma unroll
-      for (int a = 0; a < 6; ++a) cg[a] = (C)__ldg(ag.c + 6 * (size_t)(e0 + sl) + a);
+      for (int a = 0; a < 6; ++a) cg[a] = __ldg(ag.c + 6 * (size_t)(e0 + sl) + a);
       wij = __ldg(ag.w + a0) * __ldg(ag.w + a1);
     }
 #pragma unroll
@@ -784,9 +785,9 @@ __device__ __forceinline__ double axl_group(int e0, int ne, T* __restrict__ u,
       const C ur = F1[q], us = F2[q];
       C g0, g1, g2, g3, g4, g5;
       if (AFF) {
-        const C rho = (C)(wij * __ldg(ag.w + k));
-        g0 = cg[0] * rho; g1 = cg[1] * rho; g2 = cg[2] * rho;
-        g3 = cg[3] * rho; g4 = cg[4] * rho; g5 = cg[5] * rho;
+        const double rho = wij * __ldg(ag.w + k);
+        g0 = (C)(cg[0] * rho); g1 = (C)(cg[1] * rho); g2 = (C)(cg[2] * rho);
+        g3 = (C)(cg[3] * rho); g4 = (C)(cg[4] * rho); g5 = (C)(cg[5] * rho);
       } else {
         g0 = __ldg(gf + o);
         g1 = __ldg(gf + npts + o);
