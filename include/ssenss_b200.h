@@ -439,7 +439,8 @@ ssg_status ssg_server_create(int device, size_t hbm_budget, int max_active,
 /* Shared launches across requests (off by default, max_batch 1): a small
  * Helmholtz request (at most max_points points, absolute eps) at the head of
  * the queue runs together with the small Helmholtz requests of the same
- * order queued directly behind it, up to max_batch in all, as one
+ * order queued directly behind it (all on affine meshes or all on deformed
+ * ones: their operators differ), up to max_batch in all, as one
  * ssg_solve_helmholtz_segments on their concatenated meshes -- one operator
  * and one DSS launch per iteration for all of them, each with its own
  * lambda, CG scalars and stop.  The requests' resident contexts provide the

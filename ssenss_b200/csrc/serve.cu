@@ -22,7 +22,8 @@
 //   * Shared launches (ssg_server_set_batching): when the head of the queue
 //     is a small Helmholtz request and the requests right behind it are
 //     small Helmholtz requests of the same order whose meshes have idle
-//     resident contexts, up to max_batch of them run as one segmented solve
+//     resident contexts and are all affine or all deformed, up to max_batch
+//     of them run as one segmented solve
 //     (seg_solve, batch.cu): their resident level-0 data is copied device to
 //     device into one concatenated level (a per-worker arena, reused), and
 //     every operator and DSS launch of an iteration serves all of them, each
@@ -215,7 +216,9 @@ Request* admit(ssg_server* S, Resident** slot, std::vector<ssg_context*>& evict,
               x = &y;
               break;
             }
-        if (!x) break;
+        // affine and deformed meshes never share a batch: a segment's operator
+        // is then its solo operator, whoever shares the launches
+        if (!x || (!sl.empty() && !x->ctx->lev[0].aff != !sl[0]->ctx->lev[0].aff)) break;
         x->busy = true;
         b.push_back(q);
         sl.push_back(x);
@@ -385,12 +388,11 @@ ssg_status run_batch(ssg_server* S, BatchArena& A, std::vector<Request*>& b,
     A.cap_dss = cap;
   }
   cudaStream_t s = c->stream;
-  // all affine: six constants an element in place of the per-point factors
-  bool aff = true, sym = true;
-  for (Resident* r : sl) {
-    aff = aff && r->ctx->lev[0].aff;
-    sym = sym && r->ctx->lev[0].sym;
-  }
+  // affine (all or none, admit): six constants an element in place of the
+  // per-point factors
+  const bool aff = sl[0]->ctx->lev[0].aff != nullptr;
+  bool sym = true;
+  for (Resident* r : sl) sym = sym && r->ctx->lev[0].sym;
   for (size_t k = 0; k < b.size(); ++k) {
     const ssg::DevLevel& D = sl[k]->ctx->lev[0];
     const size_t P = (size_t)first[k] * nt, m = D.npts;
