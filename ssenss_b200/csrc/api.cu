@@ -334,7 +334,7 @@ static ssg_status upload_all(ssg_context* c) {
       double top = 0.0;
       for (double v : *A) top = std::max(top, std::fabs(v));
       for (int q = 0; q < n * n; ++q)
-        if (!(std::fabs((*A)[q] + (*A)[n * n - 1 - q]) <= 1e-12 * top)) d.sym = false;
+        if (!(std::fabs((*A)[q] + (*A)[n * n - 1 - q]) <= mirror_noise(n) * top)) d.sym = false;
     }
     SSG_TRY(dupload(c, &d.D, h.D.data(), h.D.size()));
     SSG_TRY(dupload(c, &d.S, h.S.data(), h.S.size()));

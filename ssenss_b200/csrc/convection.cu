@@ -577,7 +577,7 @@ bool conv_eo_split(int ni, int no, const double* A, bool anti, std::vector<doubl
   for (int o = 0; o < no; ++o)
     for (int i = 0; i < ni; ++i) {
       const double a = A[o * ni + i], b = sg * A[(no - 1 - o) * ni + ni - 1 - i];
-      if (!(std::fabs(a - b) <= 1e-13 * top)) return false;
+      if (!(std::fabs(a - b) <= mirror_noise(std::max(ni, no)) * top)) return false;
       S[o * ni + i] = 0.5 * (a + b);
     }
   for (int o = 0; o < co; ++o)

@@ -77,6 +77,13 @@ inline int ax8_fragment_index(int q) {
   return k * 64 + (4 * i + (j >> 1)) * 2 + (j & 1);
 }
 
+// How far, relative to its largest entry, a matrix on n GLL points may be from
+// its mirror image (both indices reversed) and still count as symmetric or
+// antisymmetric, so that its even / odd halves stand for it: the rounding of
+// the points, 4 eps n^2 (their distances near the ends are 1 / n^2; the
+// library's own matrices are within 2 eps).
+inline double mirror_noise(int n) { return 9e-16 * n * n; }
+
 int level_orders(int n, int* orders);
 void gll_basis(int n, double* x, double* w);
 void deriv_matrix(int n, const double* x, double* D);
