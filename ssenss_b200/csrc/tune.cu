@@ -245,7 +245,9 @@ ssg_status ssg_tuning(int n, int* ax_elements_per_block, int* dss_blocks_per_sm,
   if (n < 2 || n > SSG_MAXN) return SSG_ERR_ARG;
   // 0: the FP64 tensor-core operator (one warp per element)
   const bool dmma = n == 8;
-  if (ax_elements_per_block) *ax_elements_per_block = dmma ? 0 : ax_epb(n, true);
+  // (a plane form is only tuned for matrices without the points' symmetry)
+  const int plane = g_tune_ax_epb[n].load();
+  if (ax_elements_per_block) *ax_elements_per_block = dmma ? 0 : (plane ? plane : kAxLine);
   if (dss_blocks_per_sm) *dss_blocks_per_sm = g_tune_dss_bps[n].load() > 0 ? g_tune_dss_bps[n].load() : 8;
   if (vector_blocks_per_sm) *vector_blocks_per_sm = g_tune_vec_bps.load() > 0 ? g_tune_vec_bps.load() : kVecBpsDefault;
   return SSG_OK;
