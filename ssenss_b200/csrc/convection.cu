@@ -36,9 +36,8 @@
 //    numbers an element, and the quadrature weights fold into the projection
 //    matrix: no weight is read per point.
 //
-// Matrices without that symmetry (a caller's own arrays), dealiasing orders
-// other than 3n/2 and fields at addresses that are not 16-byte aligned run a
-// runtime-order kernel of the same arithmetic.
+// Matrices without that symmetry (a caller's own arrays) and dealiasing orders
+// other than 3n/2 run a runtime-order kernel of the same arithmetic.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -185,9 +184,11 @@ __device__ __forceinline__ void store_row(double* p, const double (&x)[L]) {
 
 // nf fields (field f at src0 for f < 3, src1 for f >= 3, components `cs`
 // apart; n^3 in global) interpolated into dst (fields FM apart), in place
-// stage by stage; ends with a barrier
+// stage by stage; vec: the sources start on 16-byte boundaries (even orders
+// then load pairs; a caller's field may not); ends with a barrier
 template <int N>
-__device__ __forceinline__ void conv_interpolate(const ConvMats<N, ConvLine<N>::M>& mt, int nf,
+__device__ __forceinline__ void conv_interpolate(const ConvMats<N, ConvLine<N>::M>& mt, bool vec,
+                                                 int nf,
                                                  const double* __restrict__ src0,
                                                  const double* __restrict__ src1, size_t cs,
                                                  double* dst) {
@@ -198,7 +199,14 @@ __device__ __forceinline__ void conv_interpolate(const ConvMats<N, ConvLine<N>::
     const int f = t / (N * N), jk = t - f * (N * N), j = jk % N, k = jk / N;
     const double* s = (f < 3 ? src0 + f * cs : src1 + (f - 3) * cs) + jk * N;
     double x[N], y[M];
-    load_row<N, N % 2 == 0>(s, x);
+    if constexpr (N % 2 == 0) {
+      if (vec)
+        load_row<N, true>(s, x);
+      else
+        load_row<N, false>(s, x);
+    } else {
+      load_row<N, false>(s, x);
+    }
     eo_contract<N, M, false>(mt.JE, mt.JO, x, y);
     store_row<M, RM % 2 == 0>(dst + f * FM + k * PL + j * RM, y);
   }
@@ -402,6 +410,7 @@ __global__ void __launch_bounds__(ConvLine<N>::THREADS, ConvLine<N>::BLOCKS)
   double* const SK = L::GSK ? scratch + (size_t)blockIdx.x * NB * FM : U + (3 + NB) * FM;
   double* const AB = U + (3 + (L::GSK ? 1 : 2) * NB) * FM;
   const bool self = u == v;
+  const bool vec = ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(v)) & 15u) == 0;
   const size_t cs = (size_t)nel * NT, ws = AFF ? 1 : (size_t)nel_fac * MT;
   for (int e = blockIdx.x; e < nel; e += gridDim.x) {
     // the next element's fields (and weights) into L2 while this one
@@ -427,17 +436,17 @@ __global__ void __launch_bounds__(ConvLine<N>::THREADS, ConvLine<N>::BLOCKS)
     double* oe = udv + (size_t)e * NT;
     if constexpr (NB == 3) {
       double* const V = self ? U : U + 3 * FM;
-      conv_interpolate<N>(mt, self ? 3 : 6, ue, ve, cs, U);
+      conv_interpolate<N>(mt, vec, self ? 3 : 6, ue, ve, cs, U);
       conv_pass<N, 0, AFF>(mt, 3, U, V, SK, AB, Wb, ws);
       conv_pass<N, 1, AFF>(mt, 3, U, V, SK, AB, Wb + 3 * ws, ws);
       conv_pass<N, 2, AFF>(mt, 3, U, V, SK, AB, Wb + 6 * ws, ws);
       conv_project<N>(mt, 3, SK, oe, cs);
     } else {
-      conv_interpolate<N>(mt, 3, ue, ue, cs, U);
+      conv_interpolate<N>(mt, vec, 3, ue, ue, cs, U);
 #pragma unroll 1
       for (int c = 0; c < 3; ++c) {
         double* const V = self ? U + c * FM : U + 3 * FM;
-        if (!self) conv_interpolate<N>(mt, 1, ve + c * cs, ve, cs, V);
+        if (!self) conv_interpolate<N>(mt, vec, 1, ve + c * cs, ve, cs, V);
         conv_pass<N, 0, AFF>(mt, 1, U, V, SK, AB, Wb, ws);
         conv_pass<N, 1, AFF>(mt, 1, U, V, SK, AB, Wb + 3 * ws, ws);
         conv_pass<N, 2, AFF>(mt, 1, U, V, SK, AB, Wb + 6 * ws, ws);
@@ -634,11 +643,7 @@ static cudaError_t launch_line(cudaStream_t s, int nel, int e0, int nel_fac, con
 cudaError_t run_convection(cudaStream_t s, int nel, int e0, int nel_fac, int n, int m,
                            const double* u, const double* v, double* udv, const ConvGeom& g) {
   if (nel <= 0) return cudaSuccess;
-  // even orders read element lines with 16-byte loads: fields at addresses
-  // that are not 16-byte aligned take the runtime-order kernel
-  const bool aligned =
-      ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(v)) & 15u) == 0;
-  if (aligned && g.eo[0] && m == (3 * n) / 2 && (n < 12 || g.scratch)) {
+  if (g.eo[0] && m == (3 * n) / 2 && (n < 12 || g.scratch)) {
     switch (n) {
 #define SSG_CONVL(NV) \
   case NV:            \
