@@ -913,13 +913,16 @@ cudaError_t cluster_cg_n(cudaStream_t s, int device, const ClusterCgRun& L, bool
                          bool* fits) {
   using C = dev::ClusterLevel<N, T>;
   auto kern = &dev::k_cluster_cg<N, T>;
+  int epc = 0;
+  bool sgeom = false;
+  const bool aff = sizeof(T) == 8 && L.ag.c;
+  // (too large for any cluster: the kernel is not loaded for it)
+  *fits = cluster_blocks<N, T>(L.nel, dev::kClusterMax, aff, &epc, &sgeom) > 0;
+  if (!*fits) return cudaSuccess;
   static ClusterAttr attr;
   int most = 0;
   cudaError_t e = attr.ensure((const void*)kern, 512, kSmemMax, device, &most);
   if (e != cudaSuccess) return e;
-  int epc = 0;
-  bool sgeom = false;
-  const bool aff = sizeof(T) == 8 && L.ag.c;
   const int cs = cluster_blocks<N, T>(L.nel, most, aff, &epc, &sgeom);
   *fits = cs > 0;
   if (!cs || !launch) return cudaSuccess;
@@ -972,13 +975,15 @@ cudaError_t cluster_cg_t(cudaStream_t s, int device, int n, const ClusterCgRun& 
 
 template <int KP>
 cudaError_t cluster_coarse_k(cudaStream_t s, int device, dev::ClusterCoarseArgs a, bool* done) {
+  *done = false;
+  if ((a.nel + dev::kClusterMax - 1) / dev::kClusterMax * 8 > KP * dev::kCoarseThreads)
+    return cudaSuccess;   // too large for any cluster: the kernel is not loaded for it
   auto kern = &dev::k_cluster_coarse<KP>;
   constexpr size_t most_smem = KP <= 2 ? 0 : (size_t)KP * dev::kCoarseThreads * 6 * 8;
   static ClusterAttr attr;
   int most = 0;
   cudaError_t e = attr.ensure((const void*)kern, dev::kCoarseThreads, most_smem, device, &most);
   if (e != cudaSuccess) return e;
-  *done = false;
   for (int cs = 1; cs <= most; cs *= 2) {
     const int epc = (a.nel + cs - 1) / cs;
     if (epc * 8 > KP * dev::kCoarseThreads) continue;
