@@ -217,6 +217,7 @@ static ssg_status upload_all(ssg_context* c) {
   c->nel = nel;
   c->nlev = H.nlev;
   c->has_walls = false;
+  c->mask_same = true;
   for (int e = 0; e < nel; ++e)
     if (H.bc[e]) c->has_walls = true;
   if ((size_t)nel * H.lev[0].nt >= (size_t)INT32_MAX)
@@ -322,6 +323,12 @@ static ssg_status upload_all(ssg_context* c) {
                   if (on) mk[e * h.nt + (k * n + j) * n + i] = 0.0;
                 }
       SSG_TRY(dupload(c, &d.mask, mk.data(), np));
+      if (l == 0) {
+        std::vector<double> copies(mk);   // unmasked copies of each node
+        host_dss(H, n, copies.data());
+        for (size_t q = 0; q < np; ++q)
+          if (copies[q] != mk[q] * mu[q]) c->mask_same = false;
+      }
     }
     {
       std::vector<int> ec;

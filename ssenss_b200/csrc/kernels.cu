@@ -23,6 +23,7 @@
 #include <cuda/atomic>
 #include <atomic>
 #include <cuda_runtime.h>
+#include <math_constants.h>
 
 #include <initializer_list>
 #include <type_traits>
@@ -881,6 +882,29 @@ __global__ void __launch_bounds__(256) k_mul(size_t npts, T* __restrict__ x,
   SSG_GRID_LOOP(q, npts) x[q] = (T)((double)x[q] * y[q]);
 }
 
+// max |f| and max |f - g| into out[0], out[1] (zeroed by the caller; bits of
+// non-negative doubles order as integers); a difference that is not a number
+// counts as infinite
+__global__ void __launch_bounds__(256) k_gap(size_t npts, const double* __restrict__ f,
+                                             const double* __restrict__ g,
+                                             unsigned long long* __restrict__ out) {
+  double top = 0.0, gap = 0.0;
+  SSG_GRID_LOOP(q, npts) {
+    const double d = fabs(f[q] - g[q]);
+    top = fmax(top, fabs(f[q]));
+    gap = fmax(gap, isnan(d) ? CUDART_INF : d);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    gap = fmax(gap, __shfl_xor_sync(0xffffffffu, gap, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(out, (unsigned long long)__double_as_longlong(top));
+    atomicMax(out + 1, (unsigned long long)__double_as_longlong(gap));
+  }
+}
+
 // one-block reduction of partials written without a counter
 __global__ void __launch_bounds__(256) k_reduce(const double* __restrict__ part, int nblk,
                                                 int nq, double* __restrict__ sums,
@@ -1354,6 +1378,15 @@ cudaError_t run_mul(cudaStream_t s, bool fp32, size_t npts, void* x, const doubl
     { SSG_COUNT(); k_mul<float><<<vec_blocks(npts), 256, 0, s>>>(npts, (float*)x, y); }
   else
     { SSG_COUNT(); k_mul<double><<<vec_blocks(npts), 256, 0, s>>>(npts, (double*)x, y); }
+  return cudaGetLastError();
+}
+
+cudaError_t run_gap(cudaStream_t s, size_t npts, const double* f, const double* g,
+                    double* out) {
+  cudaError_t e = cudaMemsetAsync(out, 0, 2 * sizeof(double), s);
+  if (e != cudaSuccess) return e;
+  SSG_COUNT();
+  k_gap<<<vec_blocks(npts), 256, 0, s>>>(npts, f, g, reinterpret_cast<unsigned long long*>(out));
   return cudaGetLastError();
 }
 

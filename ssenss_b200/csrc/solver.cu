@@ -44,10 +44,12 @@ struct Workspace {
   cudaGraphExec_t vcycle = nullptr;
   double vcycle_eps = -1.0;
   int vcycle_precision = -1;
+  bool vcycle_same = false;
   unsigned long long vcycle_kernels = 0;
   bool vcycle_failed = false;
   double warm_eps = -1.0;   // eps / precision of the last direct V-cycle
   int warm_precision = -1;
+  bool warm_same = false;
   // FCG iterations as graphs: one per window state (the slot rotation of
   // the direction history is periodic: state 0 for the first iteration,
   // then 44 states that repeat), each an IF node that runs the iteration
@@ -59,6 +61,7 @@ struct Workspace {
   double fcg_eps = -1.0;
   int fcg_precision = -1, fcg_max_iter = -1, fcg_hcap = -1;
   const double* fcg_u = nullptr;   // the solution vector the graphs update
+  bool fcg_same = false;
   bool fcg_failed = false;
   int fcg_warm = 0;          // solves run directly with this configuration
   // the Jacobi CG loop (iterations after the first) as one WHILE graph per
@@ -75,11 +78,11 @@ struct Workspace {
     const double* hist = nullptr;
     double eps = -1.0, lam = 0.0;
     int max_iter = -1, hist_cap = 0, var = -1, level = -1, frame = -1;
-    bool fp32 = false;
+    bool fp32 = false, fused = false;
     bool operator==(const LoopKey& o) const {
       return f == o.f && x == o.x && hist == o.hist && eps == o.eps && lam == o.lam &&
              max_iter == o.max_iter && hist_cap == o.hist_cap && var == o.var &&
-             level == o.level && frame == o.frame && fp32 == o.fp32;
+             level == o.level && frame == o.frame && fp32 == o.fp32 && fused == o.fused;
     }
   } cgloop_key[kLoops];
   bool cgloop_failed = false;
@@ -279,18 +282,46 @@ static ssg_status cg_outcome(ssg_context* c, const double* fr, double eps, int m
   return SSG_OK;
 }
 
-// Whether all copies of a node hold the same p in the CG of a level.  Below
-// level 0 the right-hand side is a DSS average and the start a prolonged
-// continuous field.  At level 0 the caller's right-hand side may differ
-// between copies, and where a wall meets an element in an edge alone the
-// element's copies of that edge are not masked: the FP64 solve there keeps the
-// reference's alpha, from the weighted dot of the assembled ap
-// (src/solver.c:62-65), for any input.
-static bool continuous_p(int level) { return level > 0; }
+// Whether the copies of every node hold the same value of a level-0 field, to
+// the rounding of its summation (64 eps of the largest entry; the CG's own
+// updates leave differences of that size).  A DSS, one pass and one host
+// synchronisation.
+static ssg_status same_in_copies(ssg_context* c, const double* f, bool* same) {
+  const DevLevel& L = c->lev[0];
+  double* avg = workspace_scratch(c);
+  SSG_CUDA(c, run_dss(c->stream, DSS_AVG, false, L.n, c->nel, f, avg, c->d_nbreg, L.dss_ec,
+                      nullptr, nullptr, nullptr, nullptr));
+  SSG_CUDA(c, run_gap(c->stream, L.npts, f, avg, c->d_sums));
+  SSG_CUDA(c, cudaMemcpyAsync(c->h_pin, c->d_sums, 2 * sizeof(double), cudaMemcpyDeviceToHost,
+                              c->stream));
+  SSG_CUDA(c, cudaStreamSynchronize(c->stream));
+  *same = c->h_pin[1] <= 1.4e-14 * c->h_pin[0];
+  return SSG_OK;
+}
+
+// Whether the line-run gather with the update in it may serve the FP64 CG of
+// level 0 for an unknown right-hand side f and iterate x (same_in_copies is
+// then asked): the pairing is regular, walls mask all copies of a node or none,
+// and the caller's x is on the 16-byte boundary of the vector loads.
+static bool fused_level0(const ssg_context* c, const void* x) {
+  return c->d_nbreg && c->mask_same &&
+         (c->n % 2 || reinterpret_cast<uintptr_t>(x) % 16u == 0);
+}
+
+// whether cg_solve of level 0 runs in one cluster
+static bool cluster_level0(ssg_context* c) {
+  const DevLevel& L = c->lev[0];
+  ClusterCgRun R;
+  R.nel = c->nel;
+  R.ag = aff_geom(L);
+  bool fits = false;
+  if (L.n == 8 && !R.ag.c) return false;
+  return run_cluster_cg(c->stream, c->device, L.n, false, R, false, &fits) == cudaSuccess && fits;
+}
 
 ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void* x,
                     double eps, int max_iter, int frame, double* hist, int hist_cap,
-                    bool sync_each) {
+                    bool sync_each, bool same) {
   const DevLevel& L = c->lev[level];
   LevelWork& W = fp32 ? c->ws->w32[level] : c->ws->w64[level];
   const size_t np = L.npts;
@@ -342,7 +373,7 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
     R.frame = fr;
     R.hist = hist;
     R.hist_cap = hist_cap;
-    R.weighted = !fp32 && !continuous_p(level);
+    R.weighted = !fp32 && level == 0 && !same;
     bool fits = false;
     // (n = 8 keeps its FP64 factors in fragment order: affine levels only)
     if (max_iter > 0 && (R.gf || R.ag.c))
@@ -382,13 +413,20 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
   // (p w).DSS(mask A p) = p . (mask A p) when all copies of a node hold the
   // same p, so the operator kernel reduces it, alpha is known before the DSS,
   // and the DSS gather feeds the update directly: two kernels per iteration,
-  // ap never stored.  In FP64 only where p is continuous by construction
-  // (continuous_p; Poisson solves on periodic boxes, n = 12 on 10^3 elements
-  // 19.7 -> 19.1 ms, n = 9 on 14^3 24.2 -> 23.4; level 0 in this form as well
-  // would give 18.2 and 23.7, n = 8 on 16^3 21.2 for 23.0); on meshes without
-  // the line-run DSS (irregular pairing) the FP64 gather and update stay
-  // apart, as the gather-word kernel gains nothing fused (62 us).
-  const bool fused = fp32 || (c->d_nbreg && continuous_p(level));
+  // ap never stored.  FP64 takes that form only for a p that is continuous:
+  // below level 0 it is by construction (the right-hand side is a DSS average,
+  // the start a prolonged continuous field); at level 0 the caller's
+  // right-hand side may differ between copies, and a wall that meets an element
+  // in an edge alone leaves its copies of the edge unmasked, so there it is
+  // asked (same: by the outer solve; a solve of its own asks here), and any
+  // other input keeps the reference's alpha, from the weighted dot of the
+  // assembled ap (src/solver.c:62-65).  Poisson on 16^3 elements at n = 8 23.0
+  // -> 21.2 ms, n = 12 on 10^3 19.7 -> 18.2.  On meshes without the line-run
+  // DSS (irregular pairing) the FP64 gather and update stay apart, as the
+  // gather-word kernel gains nothing fused (62 us).
+  bool fused = fp32 || (c->d_nbreg && (level > 0 || same));
+  if (!fused && level == 0 && sync_each && max_iter > 1 && fused_level0(c, x))
+    SSG_TRY(same_in_copies(c, (const double*)f, &fused));
   ScalarOp dop = op;
   if (fused) {
     pu.dot = &dop;
@@ -420,6 +458,7 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
   key.level = level;
   key.frame = frame;
   key.fp32 = fp32;
+  key.fused = fused;
   const bool loop_graph = sync_each && c->graphs && !wsp->cgloop_failed && max_iter > 1;
   for (int it = 0; it < max_iter; ++it) {
     if (loop_graph && it == 1) {
@@ -541,7 +580,7 @@ static ssg_status coarse_solve(ssg_context* c, int L, double* f, double* x, doub
 
 // V-cycle from level L (multigrid_recurse, src/precon.c:238-271)
 static ssg_status mg_recurse(ssg_context* c, int L, void* f, void* x, double eps,
-                             bool fp32) {
+                             bool fp32, bool same) {
   const int last = c->nlev - 1;
   cudaStream_t s = c->stream;
   if (L == last) {
@@ -577,7 +616,7 @@ static ssg_status mg_recurse(ssg_context* c, int L, void* f, void* x, double eps
   SSG_CUDA(c, run_dss(s, DSS_AVG, fp32, C.n, c->nel, Wc.tc, Wc.f, c->d_nbreg, C.dss_ec, nullptr,
                       nullptr, nullptr, nullptr));
   SSG_CUDA(c, cudaMemsetAsync(Wc.x, 0, C.npts * (fp32 ? sizeof(float) : sizeof(double)), s));
-  SSG_TRY(mg_recurse(c, L + 1, Wc.f, Wc.x, eps, fp32));
+  SSG_TRY(mg_recurse(c, L + 1, Wc.f, Wc.x, eps, fp32, true));
   // prolongation J^3 and x += e
   SSG_CUDA(c, run_tensor3(s, fp32, true, c->nel, C.n, F.n,
                           C.Ap, Wc.x, x));
@@ -620,12 +659,13 @@ static ssg_status mg_recurse(ssg_context* c, int L, void* f, void* x, double eps
     SSG_CUDA(c, run_level_cg(s, c->device, F.n, fp32, R));
     return SSG_OK;
   }
-  return cg_solve(c, L, SSG_PRESSURE, fp32, f, x, eps, 15, FR_LEVEL0 + L, nullptr, 0, false);
+  return cg_solve(c, L, SSG_PRESSURE, fp32, f, x, eps, 15, FR_LEVEL0 + L, nullptr, 0, false,
+                  same);
 }
 
 // z = M^-1 r: Jacobi then one V-cycle (multigrid_preconditioner,
 // src/precon.c:227-236)
-ssg_status mg_apply(ssg_context* c, const double* r, double* z, double eps) {
+ssg_status mg_apply(ssg_context* c, const double* r, double* z, double eps, bool same) {
   SSG_TRY(ensure_workspace(c));
   const bool fp32 = c->precision == SSG_PRECISION_MIXED;
   const DevLevel& L = c->lev[0];
@@ -642,7 +682,7 @@ ssg_status mg_apply(ssg_context* c, const double* r, double* z, double eps) {
   SSG_CUDA(c, run_jacobi(s, fp32, np, f0, fp32 ? (const void*)L.dinv_p32 : (const void*)L.dinv_p,
                          L.mult, x0, c->d_part,
                          nb));
-  if (c->nlev > 1) SSG_TRY(mg_recurse(c, 0, f0, x0, eps, fp32));
+  if (c->nlev > 1) SSG_TRY(mg_recurse(c, 0, f0, x0, eps, fp32, same));
   if (fp32) SSG_CUDA(c, run_convert(s, np, x0, true, z, false));
   return SSG_OK;
 }
@@ -650,18 +690,21 @@ ssg_status mg_apply(ssg_context* c, const double* r, double* z, double eps) {
 // z = M^-1 r for the FCG workspace vectors (r = ws->r, z = ws->z): replays
 // the captured V-cycle graph, capturing it on first use for this eps and
 // precision.  A capture the driver refuses falls back to direct launches.
-static ssg_status vcycle_ws(ssg_context* c, double eps) {
+static ssg_status vcycle_ws(ssg_context* c, double eps, bool same) {
   Workspace* w = c->ws;
-  if (!c->graphs || w->vcycle_failed) return mg_apply(c, w->r, w->z, eps);
+  if (!c->graphs || w->vcycle_failed) return mg_apply(c, w->r, w->z, eps, same);
   cudaStream_t s = c->stream;
-  if (w->vcycle && (w->vcycle_eps != eps || w->vcycle_precision != c->precision))
+  if (w->vcycle && (w->vcycle_eps != eps || w->vcycle_precision != c->precision ||
+                    w->vcycle_same != same))
     invalidate_graphs(c);
-  if (!w->vcycle && (w->warm_eps != eps || w->warm_precision != c->precision)) {
+  if (!w->vcycle &&
+      (w->warm_eps != eps || w->warm_precision != c->precision || w->warm_same != same)) {
     // first V-cycle of this configuration runs directly: one-time kernel
     // attribute settings happen outside any capture
     w->warm_eps = eps;
     w->warm_precision = c->precision;
-    return mg_apply(c, w->r, w->z, eps);
+    w->warm_same = same;
+    return mg_apply(c, w->r, w->z, eps, same);
   }
   if (!w->vcycle) {
     const unsigned long long before = t_launches;
@@ -669,9 +712,9 @@ static ssg_status vcycle_ws(ssg_context* c, double eps) {
     if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
       cudaGetLastError();
       w->vcycle_failed = true;
-      return mg_apply(c, w->r, w->z, eps);
+      return mg_apply(c, w->r, w->z, eps, same);
     }
-    const ssg_status st = mg_apply(c, w->r, w->z, eps);
+    const ssg_status st = mg_apply(c, w->r, w->z, eps, same);
     const cudaError_t ce = cudaStreamEndCapture(s, &g);
     const unsigned long long captured = t_launches - before;
     g_launches -= captured;   // recorded, not launched
@@ -683,12 +726,13 @@ static ssg_status vcycle_ws(ssg_context* c, double eps) {
       if (g) cudaGraphDestroy(g);
       w->vcycle_failed = true;
       c->err.clear();
-      return mg_apply(c, w->r, w->z, eps);
+      return mg_apply(c, w->r, w->z, eps, same);
     }
     cudaGraphDestroy(g);
     w->vcycle = ex;
     w->vcycle_eps = eps;
     w->vcycle_precision = c->precision;
+    w->vcycle_same = same;
     w->vcycle_kernels = captured;
   }
   SSG_CUDA(c, cudaGraphLaunch(w->vcycle, s));
@@ -721,6 +765,13 @@ ssg_status fcg_solve(ssg_context* c, const double* f, double* u, double eps, int
   op.hist = hcap ? w->hist : nullptr;
   op.hist_cap = hcap;
 
+  // the level-0 smoother's form (cg_solve): every residual is f less a
+  // continuous field
+  bool same = false;
+  if (c->precision == SSG_PRECISION_FP64 && c->nlev > 1 && fused_level0(c, nullptr) &&
+      !cluster_level0(c))
+    SSG_TRY(same_in_copies(c, f, &same));
+
   // r = f - A u; subtract_nullspace(r)
   SSG_CUDA(c, run_ax(s, L.n, c->nel, 0, false, false, u, w->aploc, L.gf, np, nullptr, L.D,
                      L.D, 0.0, nullptr, aff_geom(L)));
@@ -746,9 +797,9 @@ ssg_status fcg_solve(ssg_context* c, const double* f, double* u, double eps, int
     m = std::min(m, j);
     if (enqueue) {
       if (vcycle_graph)
-        SSG_TRY(vcycle_ws(c, eps));
+        SSG_TRY(vcycle_ws(c, eps, same));
       else
-        SSG_TRY(mg_apply(c, w->r, w->z, eps));
+        SSG_TRY(mg_apply(c, w->r, w->z, eps, same));
       // subtract_nullspace(z)
       op.code = OP_NULL_C;
       SSG_CUDA(c, run_wsum(s, false, np, w->z, L.mult, c->d_part, nb, &op));
@@ -808,7 +859,7 @@ ssg_status fcg_solve(ssg_context* c, const double* f, double* u, double eps, int
   // Iterations past the stop skip their work on the device.  Results are
   // those of the direct launches (the same kernels in the same order).
   const bool same_cfg = w->fcg_eps == eps && w->fcg_precision == c->precision &&
-                        w->fcg_max_iter == max_iter && w->fcg_hcap == hcap && w->fcg_u == u;
+                        w->fcg_max_iter == max_iter && w->fcg_hcap == hcap && w->fcg_u == u && w->fcg_same == same;
   if (!same_cfg) {
     drop_iteration_graphs(w);
     w->fcg_eps = eps;
@@ -816,6 +867,7 @@ ssg_status fcg_solve(ssg_context* c, const double* f, double* u, double eps, int
     w->fcg_max_iter = max_iter;
     w->fcg_hcap = hcap;
     w->fcg_u = u;
+    w->fcg_same = same;
   }
   const bool graph_mode = c->graphs && !w->fcg_failed && w->fcg_warm > 0 && !w->vcycle_failed;
   bool graph_mode_used = false;

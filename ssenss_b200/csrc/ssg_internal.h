@@ -203,6 +203,7 @@ struct ssg_context {
   // or corner (the line-run DSS), else null (the gather-word DSS)
   int* d_nbreg = nullptr;
   bool has_walls = false;
+  bool mask_same = true;        // level 0: all copies of a node are masked, or none
   ssg::DevLevel lev[SSG_MAXLEV];
   double* inv_mass = nullptr;   // level 0
   // dealiasing grid
@@ -318,8 +319,9 @@ ssg_status op_apply(ssg_context* c, int level, int var, bool fp32, const void* i
                     void* out, bool global);
 ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void* x,
                     double eps, int max_iter, int frame, double* hist, int hist_cap,
-                    bool sync_each);
-ssg_status mg_apply(ssg_context* c, const double* r, double* z, double eps);
+                    bool sync_each, bool same = false);
+// same: r is known to hold the same value in all copies of a node
+ssg_status mg_apply(ssg_context* c, const double* r, double* z, double eps, bool same = false);
 ssg_status fcg_solve(ssg_context* c, const double* f, double* u, double eps, int max_iter,
                      ssg_solve_info* info);
 ssg_status helmholtz_diag_update(ssg_context* c);

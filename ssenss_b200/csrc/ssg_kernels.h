@@ -205,6 +205,8 @@ cudaError_t run_mul(cudaStream_t s, bool fp32, size_t npts, void* x, const doubl
 cudaError_t run_helm_diag(cudaStream_t s, size_t npts, size_t nt, const double* kd,
                           const double* rho, const double* det, double lam, double* out);
 cudaError_t run_recip(cudaStream_t s, size_t npts, double* x);
+// out[0] = max |f|, out[1] = max |f - g| (infinite where it is not a number)
+cudaError_t run_gap(cudaStream_t s, size_t npts, const double* f, const double* g, double* out);
 cudaError_t run_reduce(cudaStream_t s, const double* part, int nblk, int nq, double* sums,
                        const ScalarOp& op);
 // post-smoother CG-Jacobi of a small level (n = 4) in one cooperative

@@ -74,3 +74,37 @@ def test_walls_that_meet_an_element_in_an_edge(shape, n, gpu_ctx_factory):
     compare(ctx, orc, O.X_VELOCITY, f)
     ctx.close()
     orc.close()
+
+
+@pytest.mark.parametrize("shape, n", [((9, 9, 9), 5), ((7, 7, 7), 8)])
+def test_forms_alternate_on_one_context(shape, n, gpu_ctx_factory):
+    """Solves that may gather and update at once (a right-hand side equal in all
+    copies) and solves that may not, in turn through the same buffers and
+    graphs: three iterations each against the oracle, and every repeat bitwise
+    the first of its kind."""
+    m = box_mesh(shape)
+    lam = 50.0
+    orc = O.Oracle(m, n)
+    orc.set_params(0.0, (11.0 / 6.0) / lam, 1.0)
+    ctx = gpu_ctx_factory(m, n, dt=(11.0 / 6.0) / lam, visc=1.0)
+    rough = ctx.level_data(0, 6) * np.random.default_rng(n).standard_normal((m.nel, n, n, n))
+    w = ctx.level_data(0, 9)
+    fs = []
+    for f in (orc.dss(rough), rough):
+        f = f - (w * f).sum() / w.sum()
+        fs.append(f)
+    z = np.zeros_like(rough)
+    ref = [[orc.solve_helmholtz(O.X_VELOCITY, f.copy(), z.copy(), eps=1e-300, max_iter=3),
+            orc.solve_poisson(f.copy(), z.copy(), eps=1e-10, max_iter=3)] for f in fs]
+    first = {}
+    for k in (0, 1, 0, 0, 1, 1, 0, 1):
+        got = [ctx.solve_helmholtz_cg(O.X_VELOCITY, fs[k], z.copy(), eps=1e-300, max_iter=3),
+               ctx.solve_poisson_cg(fs[k], z.copy(), eps=1e-10, max_iter=3)]
+        for s in range(2):
+            u, info = got[s]
+            u_o, h_o = ref[k][s]
+            assert np.all(np.abs(info["history"] - h_o) <= 1e-9 * h_o[0])
+            assert np.abs(u - u_o).max() <= 1e-8 * np.abs(u_o).max()
+            assert np.array_equal(first.setdefault((k, s), u.copy()), u)
+    ctx.close()
+    orc.close()
