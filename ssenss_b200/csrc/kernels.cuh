@@ -589,16 +589,18 @@ struct AxLine {
   static constexpr int SMEM = MATS + EPB * 3 * FS;       // values of type T
 };
 
-// Blocks an SM the line-form kernel asks for: only where the compiler's own
-// choice of registers leaves too few warps (FP64: n = 9; from n = 10 the
-// Laplacian -- n = 12 unbounded takes 216 registers, five warps an SM: 26.7
-// us on 576 affine elements, 20.6 with two blocks; n = 10 35.0 and 26.6).
-// Elsewhere the bound makes it slower (n = 7: 15.1 -> 16.4, n = 5: 15.4 ->
-// 17.5, FP32 likewise).
+// Blocks an SM the line-form kernel asks for: two, and only where the
+// compiler's own choice of registers leaves too few warps (FP64: n = 9; from
+// n = 10 the Laplacian -- n = 12 unbounded takes 216 registers, five warps an
+// SM: 26.7 us on 576 affine elements, 20.6 with two blocks; n = 10 on 1728 35.0
+// and 26.6).  Asking for more than the shared memory holds (n = 11: two) only
+// takes registers away: n = 11 with four spilled 1.4 KB a thread, 94.8 us on
+// 1728 affine elements, 39.0 with two.  Elsewhere the bound makes it slower
+// (n = 7: 15.1 -> 16.4, n = 5: 15.4 -> 17.5, FP32 likewise).
 template <int N, typename T, bool HELM>
 constexpr int axl_blocks() {
   if (sizeof(T) == 4 || N < 9 || (N >= 10 && HELM)) return 1;
-  return N == 11 ? 4 : 2;
+  return 2;
 }
 
 // y = A x; every lane of the warp reads the same entries (broadcasts of
