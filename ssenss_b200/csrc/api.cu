@@ -242,6 +242,7 @@ static ssg_status upload_all(ssg_context* c) {
         nb[26 * e + sl] = other;
       }
     if (regular) SSG_TRY(dupload(c, &c->d_nbreg, nb.data(), nb.size()));
+    c->pairs_full = dss_is_complete(H);
   }
   for (int l = 0; l < H.nlev; ++l) {
     const ssg::HostLevel& h = H.lev[l];

@@ -457,6 +457,34 @@ void dss_map_table(const HostMesh& m, int n, std::vector<int>& tab) {
   });
 }
 
+bool dss_is_complete(const HostMesh& m) {
+  // order 3 has one node inside every face and edge and at every corner; the
+  // nodes along a face or an edge pair in the same order
+  constexpr int n = 3, nt = 27;
+  std::atomic<bool> complete{true};
+  parallel_elements(m.nel, [&](int e0, int e1) {
+    // the node and its sources, sorted
+    auto copies = [&](int g, int (&c)[8]) {
+      int src[7], k = 0;
+      node_sources(m, n, g / nt, g % nt, src);
+      c[k++] = g;
+      for (int s : src)
+        if (s >= 0) c[k++] = s;
+      std::sort(c, c + k);
+      return k;
+    };
+    for (int g = e0 * nt; g < e1 * nt && complete.load(std::memory_order_relaxed); ++g) {
+      int own[8], other[8];
+      const int k = copies(g, own);
+      if (k < 2) continue;
+      for (int q = 0; q < k; ++q)
+        if (own[q] != g && (copies(own[q], other) != k || !std::equal(own, own + k, other)))
+          complete.store(false, std::memory_order_relaxed);
+    }
+  });
+  return complete.load();
+}
+
 // The factors of an affine element are one constant up to the rounding of
 // the differentiated node coordinates, relative noise of about eps |x| n^2 / h
 // (measured on boxes of 3 to 32 elements along a side: 4e-14 at n = 6, 1e-12

@@ -301,10 +301,10 @@ static ssg_status same_in_copies(ssg_context* c, const double* f, bool* same) {
 
 // Whether the line-run gather with the update in it may serve the FP64 CG of
 // level 0 for an unknown right-hand side f and iterate x (same_in_copies is
-// then asked): the pairing is regular, walls mask all copies of a node or none,
+// then asked): the pairing is regular and complete, walls mask all copies of a node or none,
 // and the caller's x is on the 16-byte boundary of the vector loads.
 static bool fused_level0(const ssg_context* c, const void* x) {
-  return c->d_nbreg && c->mask_same &&
+  return c->d_nbreg && c->pairs_full && c->mask_same &&
          (c->n % 2 || reinterpret_cast<uintptr_t>(x) % 16u == 0);
 }
 
@@ -373,7 +373,7 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
     R.frame = fr;
     R.hist = hist;
     R.hist_cap = hist_cap;
-    R.weighted = !fp32 && level == 0 && !same;
+    R.weighted = !fp32 && (!c->pairs_full || (level == 0 && !same));
     bool fits = false;
     // (n = 8 keeps its FP64 factors in fragment order: affine levels only)
     if (max_iter > 0 && (R.gf || R.ag.c))
@@ -414,8 +414,9 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
   // same p, so the operator kernel reduces it, alpha is known before the DSS,
   // and the DSS gather feeds the update directly: two kernels per iteration,
   // ap never stored.  FP64 takes that form only for a p that is continuous:
-  // below level 0 it is by construction (the right-hand side is a DSS average,
-  // the start a prolonged continuous field); at level 0 the caller's
+  // where the DSS makes a field continuous at all (pairs_full) it is so below
+  // level 0 by construction (the right-hand side is a DSS average, the start a
+  // prolonged continuous field); at level 0 the caller's
   // right-hand side may differ between copies, and a wall that meets an element
   // in an edge alone leaves its copies of the edge unmasked, so there it is
   // asked (same: by the outer solve; a solve of its own asks here), and any
@@ -424,7 +425,7 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
   // -> 21.2 ms, n = 12 on 10^3 19.7 -> 18.2.  On meshes without the line-run
   // DSS (irregular pairing) the FP64 gather and update stay apart, as the
   // gather-word kernel gains nothing fused (62 us).
-  bool fused = fp32 || (c->d_nbreg && (level > 0 || same));
+  bool fused = fp32 || (c->d_nbreg && c->pairs_full && (level > 0 || same));
   if (!fused && level == 0 && sync_each && max_iter > 1 && fused_level0(c, x))
     SSG_TRY(same_in_copies(c, (const double*)f, &fused));
   ScalarOp dop = op;
@@ -565,10 +566,12 @@ static ssg_status coarse_solve(ssg_context* c, int L, double* f, double* x, doub
     return cg_solve(c, L, SSG_PRESSURE, false, f, x, eps, max_iter, FR_LEVEL0 + L, nullptr,
                     0, false);
   }
+  // (the cluster takes p.(A p) before the DSS, the cooperative kernel after)
   bool done = false;
-  SSG_CUDA(c, run_cluster_coarse(c->stream, c->device, c->nel, f, x, (double*)W.aploc, C.gf,
-                                 C.D, C.dinv_p, c->d_pairs, C.nunique, eps, rel, max_iter,
-                                 c->d_sc + (FR_LEVEL0 + L) * F_SIZE, &done));
+  if (c->pairs_full)
+    SSG_CUDA(c, run_cluster_coarse(c->stream, c->device, c->nel, f, x, (double*)W.aploc, C.gf,
+                                   C.D, C.dinv_p, c->d_pairs, C.nunique, eps, rel, max_iter,
+                                   c->d_sc + (FR_LEVEL0 + L) * F_SIZE, &done));
   if (done) return SSG_OK;
   SSG_CUDA(c, run_coarse_cg(c->stream, c->device, c->nel, f, x, (double*)W.r, (double*)W.z,
                             (double*)W.p, (double*)W.aploc, (double*)W.ap, C.gf, C.D,

@@ -101,6 +101,11 @@ void affine_metric(const HostLevel& L, int nel, std::vector<double>& c);
 void affine_convection(const HostLevel& L, int nel, std::vector<double>& c);
 void stiffness_diagonal(const HostLevel& L, int nel, double* out);
 void host_dss(const HostMesh& m, int n, double* u);
+// Whether the sources of every node are exactly its other copies: summing makes
+// the copies equal and the weights 1 / copies add up to one.  Not so where the
+// neighbour tables leave one of several elements around an edge out, or pair
+// sides that are not the same points.
+bool dss_is_complete(const HostMesh& m);
 // DSS map of one level (one int array):
 //   [0, npts)         one gather word per local point, natural order: the
 //                     index (element * n^3 + node) of the face neighbour's
@@ -204,6 +209,7 @@ struct ssg_context {
   int* d_nbreg = nullptr;
   bool has_walls = false;
   bool mask_same = true;        // level 0: all copies of a node are masked, or none
+  bool pairs_full = true;       // dss_is_complete
   ssg::DevLevel lev[SSG_MAXLEV];
   double* inv_mass = nullptr;   // level 0
   // dealiasing grid
