@@ -17,13 +17,15 @@
 // (src/solver.c:33-81, src/precon.c:311-324) as cg_solve's kernels do it --
 // the same rounding to the storage type T, the DSS in the reference's order,
 // FP64 sums -- except that where p is the same in all copies of a node (the
-// levels below level 0; FP32 as in its kernels) p.(A p) is summed over the
-// element copies before the DSS, equal to the weighted product, so that it is
-// known at the same barrier as the operator's output; the FP64 solve of level
-// 0 takes (p w).ap of the assembled ap and one more barrier.  Every block adds
+// levels below level 0, and level 0 for a right-hand side that is; FP32 as in
+// its kernels) p.(A p) is summed over the element copies before the DSS, equal
+// to the weighted product, so that it is known at the same barrier as the
+// operator's output; other FP64 solves take (p w).ap of the assembled ap and
+// one more barrier (12 % of a Helmholtz solve).  Every block adds
 // the blocks' partial sums in rank order, so all take the same alpha, beta and
 // stop decision.
 #include <cuda_runtime.h>
+#include <math_constants.h>
 
 #include <algorithm>
 #include <atomic>
@@ -78,6 +80,7 @@ __device__ __forceinline__ void cluster_sync() {
 struct ClusterRed {
   double warp[4 * 16];
   double slot[2][4 * kClusterMax];
+  double max_warp[2 * 16], max_slot[2 * kClusterMax];   // red_max, once a launch
 };
 
 // sum of v over the warp, in every lane: two tensor-core products with ones
@@ -118,6 +121,33 @@ __device__ __forceinline__ void red_sum(const ClusterRed& s, int buf, int cs, do
     v[q] = warp_sum(lane < cs ? s.slot[buf][q * kClusterMax + lane] : 0.0);
 }
 
+// The maxima of two values a thread over the cluster: post() ends with the
+// block's sent, max() is for after a cluster_sync (once a launch).
+__device__ __forceinline__ void max_post(ClusterRed& s, double (&v)[2], int cs, uint32_t rank) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[q] = fmax(v[q], __shfl_xor_sync(0xffffffffu, v[q], o));
+    if (lane == 0) s.max_warp[q * 16 + wid] = v[q];
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    double m = 0.0;
+    for (int w = 0; w < nw; ++w) m = fmax(m, s.max_warp[lane * 16 + w]);
+    for (int b = 0; b < cs; ++b)
+      st_cluster(map_rank(smem_addr(&s.max_slot[lane * kClusterMax + rank]), b), m);
+  }
+}
+
+__device__ __forceinline__ void max_get(const ClusterRed& s, int cs, double (&v)[2]) {
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    v[q] = 0.0;
+    for (int b = 0; b < cs; ++b) v[q] = fmax(v[q], s.max_slot[q * kClusterMax + b]);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // general order: elements in shared memory, line-form operator
 // ---------------------------------------------------------------------------
@@ -138,7 +168,7 @@ struct ClusterCgArgs {
   const int* dss = nullptr;       // DSS map (dss_map_table)
   AffGeom ag;
   int helm = 0, pressure = 0;
-  int weighted = 0;               // alpha from the assembled A p
+  int weighted = 0;               // alpha from the assembled A p (kAlpha*)
   int sgeom = 0;                  // per-point factors in shared memory
   double nunique = 1.0, eps = 0.0;
   int max_iter = 0;
@@ -268,6 +298,29 @@ __global__ void __launch_bounds__(512) k_cluster_cg(ClusterCgArgs<T> a) {
   const T* const gp0 = a.sgeom ? G : a.gf + g0;           // factor c at gp0 + c * gs
   const size_t gs = a.sgeom ? (size_t)epc * NT : a.npts;
   __syncthreads();
+  // kAlphaAsk: the largest |f| and the largest difference between copies of a
+  // node (before any block masks its f); not a number counts as infinite
+  double span[2] = {0.0, 0.0};
+  if (a.weighted == kAlphaAsk) {
+    auto gap = [&](int q, int p) {
+      if (p < 0) return;
+      const double d = fabs((double)a.f[g0 + q] - (double)a.f[p]);
+      span[1] = fmax(span[1], isnan(d) ? CUDART_INF : d);
+    };
+    for (int q = tid; q < np; q += nthr) span[0] = fmax(span[0], fabs((double)a.f[g0 + q]));
+    for (int t = tid; t < ne * NF; t += nthr) {
+      const int e = t / NF;
+      gap(e * NT + class_ordered_node<N>(t - e * NF), src[t]);
+    }
+    for (int t = tid; t < ne * NE * 3; t += nthr) {
+      const int n = t / 3, e = n / NE;
+      gap(e * NT + class_ordered_node<N>(NF + n - e * NE), esrc[t]);
+    }
+    for (int t = tid; t < ne * 56; t += nthr) {
+      const int n = t / 7, e = n / 8;
+      gap(e * NT + corner_node(N, n & 7), csrc[t]);
+    }
+  }
 
   // the block's points four at a time: f(points, field positions, valid); the
   // four are read before any is written, so their chains overlap (one point
@@ -441,8 +494,14 @@ __global__ void __launch_bounds__(512) k_cluster_cg(ClusterCgArgs<T> a) {
       s[0] += (double)rv * inv_count(MU[q]);
     }
     red_post<1>(red, buf, s, cs, rank);
+    if (a.weighted == kAlphaAsk) max_post(red, span, cs, rank);
   }
   cluster_sync();
+  bool weighted = a.weighted != kAlphaPlain;
+  if (a.weighted == kAlphaAsk) {
+    max_get(red, cs, span);
+    weighted = !(span[1] <= 1.4e-14 * span[0]);
+  }
   double cz = 0.0, rdz = 0.0, beta = 0.0, err = 0.0, err0 = 0.0;
   {
     double s[1];
@@ -494,7 +553,7 @@ __global__ void __launch_bounds__(512) k_cluster_cg(ClusterCgArgs<T> a) {
     });
     __syncthreads();
     d[0] = op();
-    if (a.weighted) {
+    if (weighted) {
       // (p w).ap of the assembled ap: one more barrier
       cluster_sync();
       dss();
@@ -516,7 +575,7 @@ __global__ void __launch_bounds__(512) k_cluster_cg(ClusterCgArgs<T> a) {
       red_post<1>(red, buf, s, cs, rank);
     }
     cluster_sync();
-    if (!a.weighted) dss();
+    if (!weighted) dss();
     if (first) {
       red_sum<3>(red, buf, cs, d);
       rdz = d[1];

@@ -308,17 +308,6 @@ static bool fused_level0(const ssg_context* c, const void* x) {
          (c->n % 2 || reinterpret_cast<uintptr_t>(x) % 16u == 0);
 }
 
-// whether cg_solve of level 0 runs in one cluster
-static bool cluster_level0(ssg_context* c) {
-  const DevLevel& L = c->lev[0];
-  ClusterCgRun R;
-  R.nel = c->nel;
-  R.ag = aff_geom(L);
-  bool fits = false;
-  if (L.n == 8 && !R.ag.c) return false;
-  return run_cluster_cg(c->stream, c->device, L.n, false, R, false, &fits) == cudaSuccess && fits;
-}
-
 ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void* x,
                     double eps, int max_iter, int frame, double* hist, int hist_cap,
                     bool sync_each, bool same) {
@@ -373,7 +362,12 @@ ssg_status cg_solve(ssg_context* c, int level, int var, bool fp32, void* f, void
     R.frame = fr;
     R.hist = hist;
     R.hist_cap = hist_cap;
-    R.weighted = !fp32 && (!c->pairs_full || (level == 0 && !same));
+    // (a smoother does not ask: its residual has long been rounded unequally)
+    R.weighted = fp32                          ? kAlphaPlain
+                 : !c->pairs_full              ? kAlphaWeighted
+                 : level > 0 || same           ? kAlphaPlain
+                 : sync_each && c->mask_same   ? kAlphaAsk
+                                               : kAlphaWeighted;
     bool fits = false;
     // (n = 8 keeps its FP64 factors in fragment order: affine levels only)
     if (max_iter > 0 && (R.gf || R.ag.c))
@@ -639,7 +633,8 @@ static ssg_status mg_recurse(ssg_context* c, int L, void* f, void* x, double eps
     bool fits = false;
     SSG_CUDA(c, run_cluster_cg(s, c->device, F.n, fp32, K, false, &fits));
     if (fits)
-      return cg_solve(c, L, SSG_PRESSURE, fp32, f, x, eps, 15, FR_LEVEL0 + L, nullptr, 0, false);
+      return cg_solve(c, L, SSG_PRESSURE, fp32, f, x, eps, 15, FR_LEVEL0 + L, nullptr, 0, false,
+                      same);
     LevelCgRun R;
     R.nel = c->nel;
     R.f = f;
@@ -771,8 +766,7 @@ ssg_status fcg_solve(ssg_context* c, const double* f, double* u, double eps, int
   // the level-0 smoother's form (cg_solve): every residual is f less a
   // continuous field
   bool same = false;
-  if (c->precision == SSG_PRECISION_FP64 && c->nlev > 1 && fused_level0(c, nullptr) &&
-      !cluster_level0(c))
+  if (c->precision == SSG_PRECISION_FP64 && c->nlev > 1 && c->pairs_full && c->mask_same)
     SSG_TRY(same_in_copies(c, f, &same));
 
   // r = f - A u; subtract_nullspace(r)

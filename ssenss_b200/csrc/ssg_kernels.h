@@ -226,6 +226,11 @@ struct LevelCgRun {
   double* part = nullptr;
   size_t part_cap = 0;
 };
+// alpha of a CG iteration: from p.(A p) before the DSS, which is the weighted
+// product for a p that is the same in all copies of a node; from (p w).DSS(A p);
+// the first where the right-hand side is the same in all copies (to 64 eps of
+// its largest entry), else the second
+enum { kAlphaPlain = 0, kAlphaWeighted = 1, kAlphaAsk = 2 };
 // Jacobi CG of a small level in one thread-block cluster (cluster.cu): the
 // arithmetic of cg_solve at that level and precision.  launch false: only
 // tells whether the level fits.  fits false: nothing was launched.
@@ -242,7 +247,7 @@ struct ClusterCgRun {
   const double* mask = nullptr;
   const int* dss = nullptr;   // DSS map (dss_map_table)
   AffGeom ag;
-  int weighted = 0;           // alpha from (p w).DSS(A p): p may differ between copies
+  int weighted = 0;           // kAlpha*
   double nunique = 1.0, eps = 0.0;
   int max_iter = 0;
   double* frame = nullptr;
