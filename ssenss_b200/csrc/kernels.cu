@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(256, (N >= 10 ? 1 : 2)) k_ax(int nel, T* __res
 // interface as k_ax (optional direction update and p . (A p)).
 // ---------------------------------------------------------------------------
 template <int N, typename T, bool HELM, bool FUSEP, bool AFF>
-__global__ void __launch_bounds__(AxLine<N>::THREADS, axl_blocks<N, T, HELM>())
+__global__ void __launch_bounds__(AxLine<N>::THREADS, axl_blocks<N, T, HELM, AFF>())
     k_axl(int nel, T* __restrict__ u, T* __restrict__ au, const T* __restrict__ gf,
           size_t npts, const double* __restrict__ bj, const double* __restrict__ Dg,
           const double* __restrict__ Sg, double lambda, PUpdate pu, ScalarOp dop, AffGeom ag) {

@@ -596,9 +596,14 @@ struct AxLine {
 // and 26.6).  Asking for more than the shared memory holds (n = 11: two) only
 // takes registers away: n = 11 with four spilled 1.4 KB a thread, 94.8 us on
 // 1728 affine elements, 39.0 with two.  Elsewhere the bound makes it slower
-// (n = 7: 15.1 -> 16.4, n = 5: 15.4 -> 17.5, FP32 likewise).
-template <int N, typename T, bool HELM>
+// (n = 7: 15.1 -> 16.4, n = 5: 15.4 -> 17.5, FP32 likewise).  On deformed
+// elements the factors of a whole line are in flight, 136 to 216 registers: two
+// blocks from n = 9, also for Helmholtz (2000 elements: n = 10 65.8 -> 49.2 us;
+// 432 elements: n = 12 22.6 -> 18.5), three at n = 6 and 7 (12.3 -> 10.3 and
+// 18.5 -> 14.4, Helmholtz 14.4 -> 10.3 and 22.6 -> 16.4).
+template <int N, typename T, bool HELM, bool AFF>
 constexpr int axl_blocks() {
+  if (sizeof(T) == 8 && !AFF) return N >= 9 ? 2 : (N == 6 || N == 7 ? 3 : 1);
   if (sizeof(T) == 4 || N < 9 || (N >= 10 && HELM)) return 1;
   return 2;
 }
