@@ -184,8 +184,11 @@ __device__ __forceinline__ void store_row(double* p, const double (&x)[L]) {
 
 // nf fields (field f at src0 for f < 3, src1 for f >= 3, components `cs`
 // apart; n^3 in global) interpolated into dst (fields FM apart), in place
-// stage by stage; vec: the sources start on 16-byte boundaries (even orders
-// then load pairs; a caller's field may not); ends with a barrier
+// stage by stage; vec: the sources start on 16-byte boundaries, where even
+// orders up to 8 load pairs (n = 8 on 16^3 affine elements 314.6 us with single
+// loads, 307; a caller's field may start anywhere, and from n = 10 the second
+// form costs registers: n = 12 on 250 deformed elements 303.4 for 296.7); ends
+// with a barrier
 template <int N>
 __device__ __forceinline__ void conv_interpolate(const ConvMats<N, ConvLine<N>::M>& mt, bool vec,
                                                  int nf,
@@ -199,7 +202,7 @@ __device__ __forceinline__ void conv_interpolate(const ConvMats<N, ConvLine<N>::
     const int f = t / (N * N), jk = t - f * (N * N), j = jk % N, k = jk / N;
     const double* s = (f < 3 ? src0 + f * cs : src1 + (f - 3) * cs) + jk * N;
     double x[N], y[M];
-    if constexpr (N % 2 == 0) {
+    if constexpr (N % 2 == 0 && N <= 8) {
       if (vec)
         load_row<N, true>(s, x);
       else
