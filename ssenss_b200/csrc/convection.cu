@@ -95,6 +95,11 @@ struct ConvLine {
   // components (lines reading the weights themselves: 143.6 us a call at
   // n = 8 on 1024 deformed elements); n >= 11 has no room for them
   static constexpr bool AB = (size_t)(5 + 2 * NB) * FM * 8 <= 227 * 1024;
+  // self-convection: two such pairs by turns, the second in V's fields
+  // (conv_passes), where one block has the SM to itself (1024 deformed
+  // elements: n = 8 122.0 -> 116.4 us, n = 9 102.2 -> 94.7; below, the blocks
+  // that share an SM already overlap: n = 5 94.1 and 96.4, n = 7 112.0 and 111.3)
+  static constexpr bool TURNS = AB && NB == 3 && N >= 8;
   static constexpr size_t smem(bool aff) {
     return (size_t)(3 + (GSK ? 1 : 2) * NB + (!aff && AB ? 2 : 0)) * FM * sizeof(double);
   }
@@ -236,45 +241,52 @@ __device__ __forceinline__ void conv_interpolate(const ConvMats<N, ConvLine<N>::
   __syncthreads();
 }
 
+// A_b and B_b of a direction at every point into AB (two fields) from its three
+// per-point weight arrays Wb, `ws` apart; no barrier
+template <int N>
+__device__ __forceinline__ void conv_weights(const double* U, double* AB,
+                                             const double* __restrict__ Wb, size_t ws) {
+  using L = ConvLine<N>;
+  constexpr int M = L::M, RM = L::RM, PL = L::PL, FM = L::FM;
+  // up to six points a thread with every weight load in flight
+  constexpr int MT = M * M * M, RND = (MT + L::THREADS - 1) / L::THREADS, G = RND < 6 ? RND : 6;
+  for (int g0 = threadIdx.x; g0 < MT; g0 += G * L::THREADS) {
+    double w[G][3];
+#pragma unroll
+    for (int h = 0; h < G; ++h) {
+      const int g = g0 + h * L::THREADS;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) w[h][c] = g < MT ? __ldg(Wb + c * ws + g) : 0.0;
+    }
+#pragma unroll
+    for (int h = 0; h < G; ++h) {
+      const int g = g0 + h * L::THREADS;
+      if (g < MT) {
+        const int i = g % M, j = (g / M) % M, k = g / (M * M), q = k * PL + j * RM + i;
+        double A = w[h][0] * U[q];
+        A = fma(w[h][1], U[FM + q], A);
+        AB[q] = fma(w[h][2], U[2 * FM + q], A);
+        AB[FM + q] = (w[h][0] + w[h][1]) + w[h][2];
+      }
+    }
+  }
+}
+
 // direction B of the skew-symmetric form for nc advected components: SK_c
 // (=, +=) A_b d_b v_c + B_b d_b(u_b v_c) at every point, one line of one
-// component per thread.  AFF: cw = the element's three constants W[.][b]
-// (without the quadrature weights); else Wb = the three per-point arrays.
+// component per thread.  AFF: Wb = the element's three constants W[.][b]
+// (without the quadrature weights); else the three per-point arrays, or,
+// where they are staged, conv_weights' fields in AB.  Ends with a barrier.
 template <int N, int B, bool AFF>
 __device__ __forceinline__ void conv_pass(const ConvMats<N, ConvLine<N>::M>& mt, int nc,
                                           const double* U, const double* V, double* SK,
-                                          double* AB, const double* __restrict__ Wb,
+                                          const double* AB, const double* __restrict__ Wb,
                                           size_t ws) {
   using L = ConvLine<N>;
   constexpr int M = L::M, RM = L::RM, PL = L::PL, FM = L::FM;
   // line step in shared memory / in the unpadded global point index
   constexpr int SS = B == 0 ? 1 : (B == 1 ? RM : PL);
   constexpr int SG = B == 0 ? 1 : (B == 1 ? M : M * M);
-  if constexpr (!AFF && L::AB) {
-    // up to six points a thread with every weight load in flight
-    constexpr int MT = M * M * M, RND = (MT + L::THREADS - 1) / L::THREADS, G = RND < 6 ? RND : 6;
-    for (int g0 = threadIdx.x; g0 < MT; g0 += G * L::THREADS) {
-      double w[G][3];
-#pragma unroll
-      for (int h = 0; h < G; ++h) {
-        const int g = g0 + h * L::THREADS;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) w[h][c] = g < MT ? __ldg(Wb + c * ws + g) : 0.0;
-      }
-#pragma unroll
-      for (int h = 0; h < G; ++h) {
-        const int g = g0 + h * L::THREADS;
-        if (g < MT) {
-          const int i = g % M, j = (g / M) % M, k = g / (M * M), q = k * PL + j * RM + i;
-          double A = w[h][0] * U[q];
-          A = fma(w[h][1], U[FM + q], A);
-          AB[q] = fma(w[h][2], U[2 * FM + q], A);
-          AB[FM + q] = (w[h][0] + w[h][1]) + w[h][2];
-        }
-      }
-    }
-    __syncthreads();
-  }
   for (int t = threadIdx.x; t < nc * M * M; t += blockDim.x) {
     const int c = t / (M * M), r = t - c * (M * M);
     const int a0 = r % M, a1 = r / M;   // the two coordinates across the line
@@ -354,6 +366,33 @@ __device__ __forceinline__ void conv_pass(const ConvMats<N, ConvLine<N>::M>& mt,
     }
   }
   __syncthreads();
+}
+
+// the three directions of conv_pass with staged weights: in one pair of fields,
+// or (AB2) in two by turns, where a direction's weights form while the lines of
+// the one before are at work
+template <int N, bool AFF>
+__device__ __forceinline__ void conv_passes(const ConvMats<N, ConvLine<N>::M>& mt, int nc,
+                                            const double* U, const double* V, double* SK,
+                                            double* AB, double* AB2,
+                                            const double* __restrict__ Wb, size_t ws) {
+  constexpr bool staged = !AFF && ConvLine<N>::AB;
+  if (staged) {
+    conv_weights<N>(U, AB, Wb, ws);
+    __syncthreads();
+    if (AB2) conv_weights<N>(U, AB2, Wb + 3 * ws, ws);
+  }
+  conv_pass<N, 0, AFF>(mt, nc, U, V, SK, AB, Wb, ws);
+  if (staged) {
+    conv_weights<N>(U, AB, Wb + (AB2 ? 6 : 3) * ws, ws);
+    if (!AB2) __syncthreads();
+  }
+  conv_pass<N, 1, AFF>(mt, nc, U, V, SK, staged && AB2 ? AB2 : AB, Wb + 3 * ws, ws);
+  if (staged && !AB2) {
+    conv_weights<N>(U, AB, Wb + 6 * ws, ws);
+    __syncthreads();
+  }
+  conv_pass<N, 2, AFF>(mt, nc, U, V, SK, AB, Wb + 6 * ws, ws);
 }
 
 // nc fields of SK -> out (n^3 in global, components `cs` apart) through
@@ -440,9 +479,7 @@ __global__ void __launch_bounds__(ConvLine<N>::THREADS, ConvLine<N>::BLOCKS)
     if constexpr (NB == 3) {
       double* const V = self ? U : U + 3 * FM;
       conv_interpolate<N>(mt, vec, self ? 3 : 6, ue, ve, cs, U);
-      conv_pass<N, 0, AFF>(mt, 3, U, V, SK, AB, Wb, ws);
-      conv_pass<N, 1, AFF>(mt, 3, U, V, SK, AB, Wb + 3 * ws, ws);
-      conv_pass<N, 2, AFF>(mt, 3, U, V, SK, AB, Wb + 6 * ws, ws);
+      conv_passes<N, AFF>(mt, 3, U, V, SK, AB, L::TURNS && self ? U + 3 * FM : nullptr, Wb, ws);
       conv_project<N>(mt, 3, SK, oe, cs);
     } else {
       conv_interpolate<N>(mt, vec, 3, ue, ue, cs, U);
@@ -450,9 +487,7 @@ __global__ void __launch_bounds__(ConvLine<N>::THREADS, ConvLine<N>::BLOCKS)
       for (int c = 0; c < 3; ++c) {
         double* const V = self ? U + c * FM : U + 3 * FM;
         if (!self) conv_interpolate<N>(mt, vec, 1, ve + c * cs, ve, cs, V);
-        conv_pass<N, 0, AFF>(mt, 1, U, V, SK, AB, Wb, ws);
-        conv_pass<N, 1, AFF>(mt, 1, U, V, SK, AB, Wb + 3 * ws, ws);
-        conv_pass<N, 2, AFF>(mt, 1, U, V, SK, AB, Wb + 6 * ws, ws);
+        conv_passes<N, AFF>(mt, 1, U, V, SK, AB, nullptr, Wb, ws);
         conv_project<N>(mt, 1, SK, oe + c * cs, cs);
         // the next component's first pass writes SK, its interpolation V
         if (self) __syncthreads();
