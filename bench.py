@@ -40,13 +40,14 @@ METRIC = ("GDOF/s per PCG iter & solves/s: mixed vs FP64 GPU at 1e-10 resid; "
 UNIT = "GDOF/s"
 NE, NORD = 16, 8          # 16^3 elements, n = N + 1 = 8
 EPS = 1e-10
-# dominant kernel: the level-0 element operator (Laplacian), bytes per local
-# point: read u (8) + six G*rho*J factors (48) + write (8)
-OP_BYTES_PER_POINT = 64
+# dominant kernel: the level-0 element operator (Laplacian) on the box's affine
+# elements, bytes per local point: read u (8) + write (8), the metric six
+# constants an element (on a deformed mesh six factors a point, 48, besides)
+OP_BYTES_PER_POINT = 16
 # DRAM bytes per launch of that kernel (dram__bytes_read.sum +
 # dram__bytes_write.sum) from the ncu capture of the same workload
-# summarised in profiles/k_ax8_dmma_tgv16_n8.md
-OP_TRAFFIC_BYTES = 117918464 + 7999744
+# summarised in profiles/k_ax8_dmma_tgv16_n8.md (the result stays in L2)
+OP_TRAFFIC_BYTES = 16985600 + 0
 
 
 def parse():
@@ -683,9 +684,10 @@ def run_convection(args, ctx, mesh, n, device, calls=25):
     ms_sub, _ = cuda_timed(lib_stream, substeps, 5, 1)
     npts = mesh.nel * n ** 3
     m = (3 * n) // 2
-    # u in and udv out at n points (u == v); the nine stored weights
-    # W[a][b] = rho J tinv[a][b] / 2 at the m points
-    wbytes = 9 * 8 * mesh.nel * m ** 3
+    # u in and udv out at n points (u == v); the box's affine elements take
+    # nine constants an element for the weights (deformed ones nine values
+    # W[a][b] = rho J tinv[a][b] / 2 at each of the m^3 points)
+    wbytes = 9 * 8 * mesh.nel
     alg = (3 * 8 + 3 * 8) * npts + wbytes
     alg_gen = (6 * 8 + 3 * 8) * npts + wbytes
     return {"workload": f"TGV {args.ne}^3 N={n-1}, m={m} dealiasing grid, {calls} calls each "
@@ -1011,7 +1013,8 @@ def run_ours(args):
     alg = OP_BYTES_PER_POINT * npts
     peak, peak_kind = peaks()
     achieved = alg / (op_ms * 1e-3) / 1e9
-    # the three kernels of a smoother CG iteration at every level, each timed
+    # the three kernels of a smoother CG iteration in its assembled form (the
+    # solve's own has the update in the gather) at every level, each timed
     # alone; algorithmic bytes per point: DSS + dot 24 (in, y, out), CG update
     # 65 (x, p, r, ap, dinv, multiplicity in; x, r, z out)
     smoother = {}
@@ -1081,7 +1084,7 @@ def run_ours(args):
             "launch_shapes": ({str(k): v for k, v in tuned.items()} if tuned
                               else "default (autotuner off)"),
             "cuda_graphs": "V-cycle captured" if not args.no_graphs else "off",
-            "l2": "inputs larger than L2 (level-0 factors 100 MB + FCG vectors 420 MB)",
+            "l2": "inputs larger than L2 (FCG vectors 420 MB)",
         },
         "iterations_per_solve": it64 / args.steps,
         "solves_per_s": solves_s,
@@ -1103,12 +1106,12 @@ def run_ours(args):
                      "frac": achieved / peak,
                      "traffic": OP_TRAFFIC_BYTES if (n == 8 and args.ne == NE) else None,
                      "kernel": ("k_ax8_dmma<double> (level-0 Laplacian, FP64 DMMA)"
-                                if n == 8 else f"k_ax<{n},double> (level-0 Laplacian)"),
+                                if n == 8 else f"k_axl<{n},double> (level-0 Laplacian)"),
                      "us_per_launch": op_ms * 1e3,
                      "bytes_per_point": OP_BYTES_PER_POINT,
                      "helmholtz": {"us_per_launch": op_ms_h * 1e3,
-                                   "achieved": 72 * npts / (op_ms_h * 1e-3) / 1e9,
-                                   "frac": 72 * npts / (op_ms_h * 1e-3) / 1e9 / peak},
+                                   "achieved": 24 * npts / (op_ms_h * 1e-3) / 1e9,
+                                   "frac": 24 * npts / (op_ms_h * 1e-3) / 1e9 / peak},
                      "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)"},
         "smoother_kernels": smoother,
         "serving": serving,

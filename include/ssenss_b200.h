@@ -382,7 +382,9 @@ ssg_status ssg_autotune(ssg_context *ctx, int reps);
 ssg_status ssg_time_operator(ssg_context *ctx, int var, int reps,
 		double *us_per_apply);
 /* Device time of the three kernels of one smoother CG iteration at a
- * multigrid level, FP64, in microseconds per launch, each timed alone as
+ * multigrid level (in its assembled form: where the right-hand side is equal
+ * in all copies of a node the solves run the third inside the second), FP64,
+ * in microseconds per launch, each timed alone as
  * in ssg_time_operator (no reference counterpart: a measurement aid):
  * us[0] the element operator, us[1] the DSS with the p.(Ap) partial sums,
  * us[2] the CG update (x, r, z and four partial sums). */
