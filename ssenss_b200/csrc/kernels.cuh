@@ -571,7 +571,7 @@ struct EoMat {
 // matrices sit in shared memory and every lane of a warp reads the same
 // entries (broadcasts of pairs).  AFF: a level of affine elements reads six
 // constants an element instead of six factors a point (Helmholtz at n = 12 on
-// 576 elements, fused: 36.7 us with the factors, 26.2 without).  EPB
+// 576 elements, fused, full matrices: 36.7 us with the factors, 26.2 without).  EPB
 // elements per group fill about 256 threads.  The arithmetic runs in the
 // storage type T: FP64 for the solves, FP32 in the mixed-precision V-cycle
 // (the fused direction update and the p . (A p) sum stay FP64, and a factor of
