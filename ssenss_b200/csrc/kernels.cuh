@@ -601,9 +601,13 @@ struct AxLine {
 // blocks from n = 9, also for Helmholtz (2000 elements: n = 10 65.8 -> 49.2 us;
 // 432 elements: n = 12 22.6 -> 18.5), three at n = 6 and 7 (12.3 -> 10.3 and
 // 18.5 -> 14.4, Helmholtz 14.4 -> 10.3 and 22.6 -> 16.4).
+// FP32 on affine elements holds the six FP64 constants: three blocks where they
+// would leave two (a V-cycle on 15^3 elements at n = 7 1637 -> 1530 us, 18^3 at
+// n = 6 2151 -> 2065, 9^3 at n = 12 1661 -> 1545).
 template <int N, typename T, bool HELM, bool AFF>
 constexpr int axl_blocks() {
   if (sizeof(T) == 8 && !AFF) return N >= 9 ? 2 : (N == 6 || N == 7 ? 3 : 1);
+  if (sizeof(T) == 4 && AFF) return N == 6 || N == 7 || N == 12 ? 3 : 1;
   if (sizeof(T) == 4 || N < 9 || (N >= 10 && HELM)) return 1;
   return 2;
 }
