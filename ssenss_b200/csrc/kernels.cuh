@@ -576,7 +576,7 @@ struct EoMat {
 // storage type T: FP64 for the solves, FP32 in the mixed-precision V-cycle
 // (the fused direction update and the p . (A p) sum stay FP64, and a factor of
 // an affine element is one rounding of its FP64 value, as the stored ones are:
-// the FP32 products instead would save 1 % of a mixed solve).
+// the FP32 products instead would save 1 to 3 % of a mixed V-cycle).
 // ---------------------------------------------------------------------------
 template <int N>
 struct AxLine {
